@@ -34,6 +34,7 @@ struct DevSys {
   float inv_diag[3];  // 1/a_x, 1/b_y, 1/c_z for the minimum image
   float cutoff, cutoff2, list_cutoff, list_cutoff2;
   float alpha;
+  float pme_factor, pme_pref;  // pi^2 / alpha^2 and k_e / (pi V) of the convolution (set with the box)
   int atom_start, atom_count;
   int type_count, lj_base;
   int cell_counts[3];

@@ -23,6 +23,7 @@
 
 #include "../../include/rmd.h"
 #include "common.cuh"
+#include "fft.cuh"
 #include "kernels.h"
 
 namespace rmd {
@@ -239,8 +240,11 @@ struct Engine {
   DevArray<float2> half, twiddles;
   DevArray<float> real_grid, moduli;
   DevArray<FftPlan> fft_plans;
-  DevArray<FftTask> tasks_z, tasks_y, tasks_x, tasks_plane, tasks_cluster, tasks_y_all, tasks_x_all;
+  DevArray<FftTask> tasks_z, tasks_y, tasks_x, tasks_y_all, tasks_x_all;
+  DevArray<FftZTask> tasks_z2;
+  DevArray<FftPlaneTask> tasks_plane, tasks_cluster;
   std::vector<long long> recip_lo, recip_hi;  // per system range [lo, hi) of reciprocal energy partials
+  int fft_large = 0, z2_threads = 0, z2_smem = 0, plane_threads = 0, cluster_threads = 0;
   int plane_stride = 0, cluster_rows = 0, cluster_cols = 0;
   DevArray<DevSys> sys;
   DevArray<DevSysD> sysd;
@@ -482,7 +486,7 @@ static FastDiv make_fast_div(uint32_t d) {
   uint32_t shift = 0;
   while ((1ull << shift) < d) ++shift;
   const unsigned long long magic = (((1ull << 32) * ((1ull << shift) - d)) / d) + 1;
-  return FastDiv{(uint32_t)magic, shift};
+  return FastDiv{(uint32_t)magic, shift, (int)d};
 }
 
 static void fft_axis_plan(int n, FftAxis &ax, int tw_base) {
@@ -502,6 +506,12 @@ static void fft_axis_plan(int n, FftAxis &ax, int tw_base) {
   }
   ax.n_div = make_fast_div((uint32_t)n);
   ax.half_div = make_fast_div((uint32_t)(n / 2 + 1));
+  ax.r1 = ax.r2 = 0;
+  if (n > FFT_TWO_MAX || !fft_two_factors(n, &ax.r1, &ax.r2)) ax.r1 = ax.r2 = 0;
+}
+
+static FftTwo fft_two(const FftAxis &ax) {
+  return FftTwo{ax.n, ax.r1, ax.r2, ax.tw_base, make_fast_div((uint32_t)ax.r1), make_fast_div((uint32_t)ax.r2), ax.n_div};
 }
 
 constexpr int FFT_SMEM_HOST = 2048;
@@ -971,7 +981,9 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
     std::vector<float> h_mod;
     std::vector<float2> h_tw;
     std::vector<FftPlan> h_plans(S);
-    std::vector<FftTask> tz, ty, tx, tp, tq, ty_all, tx_all;
+    std::vector<FftTask> tz, ty, tx, ty_all, tx_all;
+    std::vector<FftZTask> tz2;
+    std::vector<FftPlaneTask> tp, tq;
     std::vector<int> split(S);
     plane_stride = cluster_rows = cluster_cols = 0;
     // Lines per block. The z and y passes (no sums across lines) are sized from the whole
@@ -1000,10 +1012,11 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
       d.half_base = hbase;
       d.moduli_base = (int)h_mod.size();
       gbase += (long long)nx * ny * nz;
-      hbase += (long long)nx * ny * nzh;
+      hbase += ((long long)nx * ny * nzh + 1) / 2 * 2;  // (every system's half spectrum starts on 16 bytes)
       for (int ax = 0; ax < 3; ++ax) {
         for (double m : bspline_moduli(h.grid[ax], h.order)) h_mod.push_back((float)m);
         fft_axis_plan(h.grid[ax], h_plans[s].axis[ax], (int)h_tw.size());
+        if (h_plans[s].axis[ax].r2 > RADIX_SMALL) fft_large = 1;
         for (int k = 0; k < h.grid[ax]; ++k) {
           const double a = -2.0 * M_PI * k / h.grid[ax];
           h_tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
@@ -1011,31 +1024,53 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
       }
       // z pass: pairs of real lines
       const int lines = nx * ny, pairs = (lines + 1) / 2;
-      const int mz = lines_per_block(all_pairs, nz, 64);
-      for (int p = 0; p < pairs; p += mz) tz.push_back(FftTask{s, 0, p, std::min(mz, pairs - p)});
+      const FftAxis &zax = h_plans[s].axis[2];
+      const int mz = zax.r1 > 0 ? FFT_PAIRS_PER_BLOCK : lines_per_block(all_pairs, nz, 64);
+      for (int p = 0; p < pairs; p += mz) {
+        if (zax.r1 > 0)
+          tz2.push_back(FftZTask{d.grid_base, d.half_base, p, std::min(mz, pairs - p), lines, fft_two(zax)});
+        else
+          tz.push_back(FftTask{s, 0, p, std::min(mz, pairs - p)});
+      }
+      if (zax.r1 > 0) {
+        z2_threads = std::max(z2_threads, std::min(256, (FFT_PAIRS_PER_BLOCK * zax.r2 + 31) / 32 * 32));
+        z2_smem = std::max(z2_smem, FFT_PAIRS_PER_BLOCK * ((zax.r1 * (zax.r2 | 1)) | 1));
+      }
       // A system whose kz plane fits shared memory runs the fused y-x-convolve-x-y pass, one
       // block or one cluster of blocks a plane; the others run the separate y and x passes. The
       // debug transforms run the separate passes over every system.
       split[s] = fft_plane_split(nx, ny);
       const bool fused = split[s] > 0;
-      const int my = lines_per_block(all_ylines, ny + 1, nzh);  // y and x lines are padded to n + 1
-      const int mx = std::max(1, std::min(nzh, std::min(FFT_SMEM_HOST / (nx + 1), 512 / (nx + 1))));
-      for (int x = 0; x < nx; ++x)
-        for (int k = 0; k < nzh; k += my) {
-          ty_all.push_back(FftTask{s, x, k, std::min(my, nzh - k)});
+      // separate passes: y lines are the x rows of a plane, x lines its columns (padded to nx + 1)
+      const int my = lines_per_block(all_ylines, ny, nx);
+      const int mx = std::max(1, std::min(ny, std::min(FFT_SMEM_HOST / (nx + 1), 512 / (nx + 1))));
+      for (int kz = 0; kz < nzh; ++kz) {
+        for (int x = 0; x < nx; x += my) {
+          ty_all.push_back(FftTask{s, kz, x, std::min(my, nx - x)});
           if (!fused) ty.push_back(ty_all.back());
         }
-      for (int y = 0; y < ny; ++y)
-        for (int k = 0; k < nzh; k += mx) {
-          tx_all.push_back(FftTask{s, y, k, std::min(mx, nzh - k)});
+        for (int y = 0; y < ny; y += mx) {
+          tx_all.push_back(FftTask{s, kz, y, std::min(mx, ny - y)});
           if (!fused) tx.push_back(tx_all.back());
         }
+      }
       int rows = 0, cols = 0;
       if (fused) fft_plane_buffers(nx, ny, split[s], &rows, &cols);
-      std::vector<FftTask> &planes = split[s] == 1 ? tp : tq;
-      for (int kz = 0; fused && kz < nzh; ++kz) planes.push_back(FftTask{s, kz, 0, 0});
-      if (split[s] == 1) plane_stride = std::max(plane_stride, rows);
+      std::vector<FftPlaneTask> &planes = split[s] == 1 ? tp : tq;
+      const int threads = fused ? fft_plane_threads(nx, ny, split[s]) : 0;
+      for (int kz = 0; fused && kz < nzh; ++kz) {
+        const FftTwo x = fft_two(h_plans[s].axis[0]), y = fft_two(h_plans[s].axis[1]);
+        planes.push_back(FftPlaneTask{d.half_base + (long long)kz * nx * ny, s, kz, nz, d.moduli_base, threads, x, y,
+                                      make_fast_div((uint32_t)((nx + split[s] - 1) / split[s])),
+                                      make_fast_div((uint32_t)((ny + split[s] - 1) / split[s])),
+                                      make_fast_div((uint32_t)(y.r1 * (y.r2 | 1)))});
+      }
+      if (split[s] == 1) {
+        plane_stride = std::max(plane_stride, rows);
+        plane_threads = std::max(plane_threads, threads);
+      }
       if (split[s] > 1) {
+        cluster_threads = std::max(cluster_threads, threads);
         cluster_rows = std::max(cluster_rows, rows);
         cluster_cols = std::max(cluster_cols, cols);
       }
@@ -1067,6 +1102,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
     moduli.upload(h_mod);
     twiddles.upload(h_tw);
     fft_plans.upload(h_plans);
+    tasks_z2.upload(tz2);
     tasks_z.upload(tz);
     tasks_y.upload(ty);
     tasks_x.upload(tx);
@@ -1317,6 +1353,13 @@ LaunchCtx Engine::ctx() const {
   c.moduli = moduli.p;
   c.twiddles = twiddles.p;
   c.fft_plans = fft_plans.p;
+  c.tasks_z2 = tasks_z2.p;
+  c.n_tasks_z2 = (int)tasks_z2.n;
+  c.fft_large = fft_large;
+  c.z2_threads = z2_threads;
+  c.z2_smem = z2_smem;
+  c.plane_threads = plane_threads;
+  c.cluster_threads = cluster_threads;
   c.tasks_z = tasks_z.p;
   c.tasks_y = tasks_y.p;
   c.tasks_x = tasks_x.p;
@@ -2746,9 +2789,11 @@ rmd_status rmd_debug_read(rmd_sim *sim, int32_t s, int32_t which, double *out) {
     } else if (which == 1) {  // half spectrum
       std::vector<float2> g(hp);
       CUDA_OK(cudaMemcpy(g.data(), e.half.p + ds.half_base, sizeof(float2) * hp, cudaMemcpyDeviceToHost));
+      const size_t nzh = h.grid[2] / 2 + 1, plane = hp / nzh;  // stored kz plane by plane
       for (size_t k = 0; k < hp; ++k) {
-        out[2 * k] = g[k].x;
-        out[2 * k + 1] = g[k].y;
+        const float2 v = g[(k % nzh) * plane + k / nzh];
+        out[2 * k] = v.x;
+        out[2 * k + 1] = v.y;
       }
     } else if (which == 2) {  // the positions the current neighbour list was built from
       std::vector<float4> o(h.n);
@@ -3022,9 +3067,11 @@ rmd_status rmd_debug_fft(rmd_sim *sim, int32_t s, const double *data, double *ha
     e.sync();
     std::vector<float2> hs_(hp);
     CUDA_OK(cudaMemcpy(hs_.data(), e.half.p + ds.half_base, sizeof(float2) * hp, cudaMemcpyDeviceToHost));
+    const size_t plane = (size_t)nx * ny;  // stored kz plane by plane
     for (size_t k = 0; k < hp; ++k) {
-      half_spectrum[2 * k] = hs_[k].x;
-      half_spectrum[2 * k + 1] = hs_[k].y;
+      const float2 v = hs_[(k % nzh) * plane + k / nzh];
+      half_spectrum[2 * k] = v.x;
+      half_spectrum[2 * k + 1] = v.y;
     }
     rmd::launch_fft_inverse(c, e.stream);
     e.sync();

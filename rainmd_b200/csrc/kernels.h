@@ -16,6 +16,7 @@ namespace rmd {
 // umulhi(x, magic) < x < 2^31).
 struct FastDiv {
   uint32_t magic, shift;
+  int d;  // the divisor
 };
 struct FftAxis {
   int n;
@@ -25,10 +26,31 @@ struct FftAxis {
   FastDiv per_line[12];  // stage s: n / radix[s] butterflies a line
   FastDiv span[12];      // stage s: the product of the earlier radices
   FastDiv n_div, half_div;  // n and n / 2 + 1
+  int r1, r2;               // n = r1 * r2 for the two-factor passes (fft.cuh); 0 when n has no such factors
 };
 struct FftPlan {
   FftAxis axis[3];
 };
+// An axis of a two-factor pass, and the passes' tasks. A task holds all that its block needs of the
+// plan, so it is one read, and nothing in it changes after the engine is built.
+struct FftTwo {
+  int n, r1, r2, tw_base;
+  FastDiv r1_div, r2_div, n_div;
+};
+struct FftZTask {
+  long long grid_base, half_base;
+  int first, count, plane;  // pairs [first, first + count) of the plane's lines; plane = nx * ny
+  FftTwo z;
+};
+struct FftPlaneTask {
+  long long half_base;      // of this kz plane
+  int sys, kz, nz, moduli_base, threads;
+  FftTwo x, y;
+  FastDiv rows_div, cols_div, ldy_div;  // rows and columns a block of the cluster; a row's padded length
+};
+constexpr int FFT_TWO_MAX = 400;          // longest axis of the two-factor passes (20 x 20)
+constexpr int FFT_PAIRS_PER_BLOCK = 8;    // pairs of real z lines a two-factor z block transforms
+constexpr int FFT_PLANE_THREADS = 512;    // most threads of a plane block
 // A block's share of an FFT pass: lines [first, first+count) of system `sys`; `fixed` is
 // the other fixed index (x for the y pass, y for the x pass).
 struct FftTask {
@@ -163,12 +185,18 @@ struct LaunchCtx {
   const float *moduli;
   const float2 *twiddles;
   const FftPlan *fft_plans;
-  // z tasks cover every system; y and x tasks the systems on the separate passes; plane tasks
+  // z2 tasks cover the systems whose z axis has two factors, z tasks the others; y and x tasks the
+  // systems on the separate passes; plane tasks
   // (one per kz plane) the systems whose planes a block transforms alone, cluster tasks (one
   // per kz plane) those whose planes a cluster of PLANE_CLUSTER blocks shares; *_all cover
   // every system (the debug transforms)
-  const FftTask *tasks_z, *tasks_y, *tasks_x, *tasks_plane, *tasks_cluster, *tasks_y_all, *tasks_x_all;
-  int n_tasks_z, n_tasks_y, n_tasks_x, n_tasks_plane, n_tasks_cluster, n_tasks_y_all, n_tasks_x_all;
+  const FftZTask *tasks_z2;
+  const FftPlaneTask *tasks_plane, *tasks_cluster;
+  const FftTask *tasks_z, *tasks_y, *tasks_x, *tasks_y_all, *tasks_x_all;
+  int n_tasks_z2, n_tasks_z, n_tasks_y, n_tasks_x, n_tasks_plane, n_tasks_cluster, n_tasks_y_all, n_tasks_x_all;
+  int fft_large;            // some axis has a factor above RADIX_SMALL
+  int z2_threads, z2_smem;  // block size and complex values of shared memory of the two-factor z passes
+  int plane_threads, cluster_threads;  // block sizes of the plane passes
   int plane_stride;  // complex values per plane buffer (the largest plane among the one-block systems)
   int cluster_rows, cluster_cols;  // complex values per row / column buffer of a cluster block
   // energy partials: one per x task, then one per plane task, then PLANE_CLUSTER per cluster task
@@ -204,9 +232,9 @@ int pme_launches(const LaunchCtx &c);  // kernels launch_pme issues
 constexpr long long FFT_PLANE_SMEM_MAX = 200 * 1024;
 constexpr int PLANE_CLUSTER = 4;
 int fft_plane_split(int nx, int ny);
-// complex values per shared buffer for a split: the whole padded plane for 1; for a cluster,
-// a block's rows (rows_per x (ny + 1)) and its columns (cols_per x (nx + 1))
+// complex values per shared buffer of a plane block: its (padded) rows, and in a cluster its columns
 void fft_plane_buffers(int nx, int ny, int split, int *rows, int *cols);
+int fft_plane_threads(int nx, int ny, int split);
 cudaError_t fft_plane_prepare();
 void launch_fft_forward(const LaunchCtx &c, cudaStream_t stream);
 void launch_spread_only(const LaunchCtx &c, cudaStream_t stream);

@@ -9,77 +9,36 @@
 // B200 design (not the reference's pass structure):
 //   spread   ORDER^2 threads per atom, 64-bit fixed-point integer atomics (deterministic);
 //   z pass   R2C: two real z-lines packed as one complex line, FFT in shared memory,
-//            split into two half spectra; also converts fixed point -> f32 and zeroes the
-//            fixed grid for the next step (no separate clear/convert kernels);
-//   y pass   complex FFT along y on the half spectrum, in place;
-//   x pass   forward FFT along x, the Ewald convolution and the FP64 energy partial, and
-//            the inverse FFT along x, all while the lines are in shared memory;
-//   y pass   inverse; z pass C2R back to a real f32 grid; gather four threads per atom.
-//   planes   where a kz plane fits shared memory, the y pass, the x pass and the inverse y
-//            pass are one kernel over whole planes: one block a plane for small planes, a
-//            thread-block cluster a plane (distributed shared memory) for larger ones.
-// Lines filled by a transpose (y and x passes) are padded to n + 1 in shared memory.
-// The FFT is a mixed-radix (4, 2, 3, 5) Stockham autosort over lines held in shared
-// memory; a host-built task table gives each block a set of lines of one system, so
+//            split into two half spectra, stored plane by plane (kz outermost); also converts
+//            fixed point -> f32 and zeroes the fixed grid for the next step;
+//   planes   forward y and x FFTs, the Ewald convolution (with the FP64 energy partial) and the
+//            inverse x and y FFTs of a whole kz plane in one kernel: one block a plane for small
+//            planes, a thread-block cluster a plane (distributed shared memory) for larger ones;
+//   z pass   C2R back to a real f32 grid; gather four threads per atom.
+// Lines are transformed by two register-resident DFTs a point (fft.cuh). Measured on one B200,
+// the reciprocal kernels run back to back, against the radix-4 Stockham passes over a spectrum
+// with kz innermost that these replaced: 32^3 27.9 -> 22.8 us, 64^3 49.2 -> 38.2, 108^3
+// 139 -> 80, 144^3 360 -> 170, a batch of 24 grids of 24^3-48^3 106 -> 80. What they gained from:
+// a plane's rows are contiguous (they were strided by the kz lines: one 32-byte sector a value),
+// the r2c pass issues all its loads before it clears the grid, and a transform is two steps
+// instead of three or four.
+// Planes beyond the cluster's shared memory, and axes without two factors (243, 384 and those
+// above 400 points), take passes of their own, y, x with the convolution, y (and z), with a
+// mixed-radix (4, 2, 3, 5) Stockham autosort; lines filled by a transpose are padded to n + 1.
+// A host-built task table gives each block a set of lines (or a plane) of one system, so
 // systems with different grid sizes run in the same launch.
 #include <algorithm>
+#include <climits>
 
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "fft.cuh"
 #include "kernels.h"
 
 namespace rmd {
 
 namespace cg = cooperative_groups;
-
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-// multiply by -i (forward) or +i (inverse)
-__device__ __forceinline__ float2 rot(float2 a, bool inverse) {
-  return inverse ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
-}
-
-template <int R>
-__device__ __forceinline__ void dft_small(float2 *v, bool inv) {
-  if (R == 2) {
-    float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-  } else if (R == 4) {
-    float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
-    float2 a2 = cadd(v[1], v[3]), a3 = rot(csub(v[1], v[3]), inv);
-    v[0] = cadd(a0, a2);
-    v[2] = csub(a0, a2);
-    v[1] = cadd(a1, a3);
-    v[3] = csub(a1, a3);
-  } else if (R == 3) {
-    const float h = 0.86602540378443864676f;  // sqrt(3)/2
-    float2 t1 = cadd(v[1], v[2]), t2 = csub(v[1], v[2]);
-    float2 b = make_float2(v[0].x - 0.5f * t1.x, v[0].y - 0.5f * t1.y);
-    float2 r = rot(make_float2(h * t2.x, h * t2.y), inv);  // -i*h*t2 forward
-    v[0] = cadd(v[0], t1);
-    v[1] = cadd(b, r);
-    v[2] = csub(b, r);
-  } else if (R == 5) {
-    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
-    const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
-    float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
-    float2 t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-    float2 b1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    float2 b2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    float2 q1 = rot(make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y), inv);
-    float2 q2 = rot(make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y), inv);
-    v[0] = cadd(v[0], cadd(t1, t2));
-    v[1] = cadd(b1, q1);
-    v[4] = csub(b1, q1);
-    v[2] = cadd(b2, q2);
-    v[3] = csub(b2, q2);
-  }
-}
 
 __device__ __forceinline__ int fast_div(int x, FastDiv f) {
   return (int)((__umulhi((uint32_t)x, f.magic) + (uint32_t)x) >> f.shift);
@@ -236,8 +195,8 @@ __global__ void __launch_bounds__(256) k_fft_z_r2c(const FftTask *__restrict__ t
     // A = (Z + conj(Zc))/2, B = -i (Z - conj(Zc))/2
     const float2 a = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 b = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
-    h[(long long)l * nzh + k] = a;
-    if (l + 1 < nlines) h[(long long)(l + 1) * nzh + k] = b;
+    h[(long long)k * nlines + l] = a;
+    if (l + 1 < nlines) h[(long long)k * nlines + l + 1] = b;
   }
 }
 
@@ -263,15 +222,15 @@ __global__ void __launch_bounds__(256) k_fft_z_c2r(const FftTask *__restrict__ t
     const bool has_b = l + 1 < nlines;
     float2 a, b;
     if (k < nzh) {
-      a = h[(long long)l * nzh + k];
-      b = has_b ? h[(long long)(l + 1) * nzh + k] : make_float2(0.f, 0.f);
+      a = h[(long long)k * nlines + l];
+      b = has_b ? h[(long long)k * nlines + l + 1] : make_float2(0.f, 0.f);
       if (k == 0 || 2 * k == N) {
         a.y = 0.f;
         b.y = 0.f;
       }
     } else {
-      a = h[(long long)l * nzh + (N - k)];
-      b = has_b ? h[(long long)(l + 1) * nzh + (N - k)] : make_float2(0.f, 0.f);
+      a = h[(long long)(N - k) * nlines + l];
+      b = has_b ? h[(long long)(N - k) * nlines + l + 1] : make_float2(0.f, 0.f);
       a.y = -a.y;
       b.y = -b.y;
     }
@@ -289,6 +248,7 @@ __global__ void __launch_bounds__(256) k_fft_z_c2r(const FftTask *__restrict__ t
 }
 
 // ------------------------------------------------------ y pass (either direction, in place)
+// A task is `count` consecutive x rows of plane kz = `fixed`: one contiguous run of the plane.
 __global__ void __launch_bounds__(256) k_fft_y(const FftTask *__restrict__ tasks,
                                                const DevSys *__restrict__ sys,
                                                const FftPlan *__restrict__ plans,
@@ -299,18 +259,65 @@ __global__ void __launch_bounds__(256) k_fft_y(const FftTask *__restrict__ tasks
   const FftTask t = tasks[blockIdx.x];
   const DevSys &s = sys[t.sys];
   const FftPlan &pl = plans[t.sys];
-  const int ny = s.grid[1], nzh = s.grid[2] / 2 + 1;
-  const int x = t.fixed, kz0 = t.first, M = t.count;
-  float2 *h = half + s.half_base + (long long)x * ny * nzh + kz0;
-  const int ld = ny + 1;  // padded lines (bank-conflict-free transpose)
-  for (int idx = threadIdx.x; idx < ny * M; idx += blockDim.x) {
-    const int y = idx / M, m = idx - y * M;
-    bufa[m * ld + y] = h[(long long)y * nzh + m];
+  const int nx = s.grid[0], ny = s.grid[1], M = t.count;
+  float2 *h = half + s.half_base + ((long long)t.fixed * nx + t.first) * ny;
+  for (int idx = threadIdx.x; idx < ny * M; idx += blockDim.x) bufa[idx] = h[idx];
+  float2 *r = fft_lines(bufa, bufb, M, ny, ny, pl.axis[1], twiddles + pl.axis[1].tw_base, inverse != 0);
+  for (int idx = threadIdx.x; idx < ny * M; idx += blockDim.x) h[idx] = r[idx];
+}
+
+// The Ewald convolution along a line of kx at fixed ky and kz (signed frequencies): the wave
+// vector is (kx, ky, kz) times the rows of the inverse box, of which the entries above the diagonal
+// are zero (the box is reduced), so only its kx part changes along the line. mod_yz: the product
+// of the y and z moduli. With ENERGY the point's energy and virial terms are added; `weight` counts
+// the point and its mirror image. The zero wave vector gives zero.
+struct ConvolveLine {
+  float r0, r3, r6, cy, cz, mod_yz, factor, pref;
+  __device__ __forceinline__ ConvolveLine(const DevSys &s, int ky, int kz, float mod) {
+    r0 = s.recip[0];
+    r3 = s.recip[3];
+    r6 = s.recip[6];
+    cy = (float)ky * s.recip[4];
+    cz = (float)ky * s.recip[7] + (float)kz * s.recip[8];
+    mod_yz = mod;
+    factor = s.pme_factor;
+    pref = s.pme_pref;
   }
-  float2 *r = fft_lines(bufa, bufb, M, ny, ld, pl.axis[1], twiddles + pl.axis[1].tw_base, inverse != 0);
-  for (int idx = threadIdx.x; idx < ny * M; idx += blockDim.x) {
-    const int y = idx / M, m = idx - y * M;
-    h[(long long)y * nzh + m] = r[m * ld + y];
+  template <bool ENERGY>
+  __device__ __forceinline__ void apply(float2 &v, int kx, float mod_x, double weight, double &energy,
+                                        double &virial) const {
+    const float fx = (float)kx;
+    const float x = fx * r0, y = fmaf(fx, r3, cy), z = fmaf(fx, r6, cz);
+    const float m2 = x * x + y * y + z * z;
+    const float kernel = m2 != 0.f ? __expf(-factor * m2) / (m2 * (mod_x * mod_yz)) : 0.f;
+    if (ENERGY) {
+      const double ek = weight * 0.5 * (double)pref * (double)kernel * ((double)v.x * v.x + (double)v.y * v.y);
+      energy += ek;
+      virial += ek * (1.0 + (double)factor * (double)m2);
+    }
+    const float sc = kernel * pref;
+    v = make_float2(v.x * sc, v.y * sc);
+  }
+};
+
+// Block sum of a thread's energy and virial terms, written by thread 0 to e[slot], ev[slot].
+__device__ __forceinline__ void block_energy(double energy, double virial, double *e, double *ev, int slot) {
+  __shared__ double red[2][32];
+  energy = warp_sum(energy);
+  virial = warp_sum(virial);
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = energy;
+    red[1][threadIdx.x >> 5] = virial;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double total = 0, total_vir = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+      total += red[0][w];
+      total_vir += red[1][w];
+    }
+    e[slot] = total;
+    ev[slot] = total_vir;
   }
 }
 
@@ -318,7 +325,6 @@ __global__ void __launch_bounds__(256) k_fft_y(const FftTask *__restrict__ tasks
 template <bool ENERGY>
 __global__ void __launch_bounds__(256) k_fft_x_convolve(const FftTask *__restrict__ tasks,
                                                         const DevSys *__restrict__ sys,
-                                                        const DevSysD *__restrict__ sysd,
                                                         const FftPlan *__restrict__ plans,
                                                         const float2 *__restrict__ twiddles,
                                                         const float *__restrict__ moduli,
@@ -327,125 +333,394 @@ __global__ void __launch_bounds__(256) k_fft_x_convolve(const FftTask *__restric
                                                         double *__restrict__ e_pme_vir) {
   chain_begin();
   __shared__ float2 bufa[FFT_SMEM], bufb[FFT_SMEM];
-  __shared__ double red[2][256 / 32];
   const FftTask t = tasks[blockIdx.x];
   const DevSys &s = sys[t.sys];
   const FftPlan &pl = plans[t.sys];
-  const int nx = s.grid[0], ny = s.grid[1], nz = s.grid[2], nzh = nz / 2 + 1;
-  const int y = t.fixed, kz0 = t.first, M = t.count;
-  const long long stride = (long long)ny * nzh;
-  float2 *h = half + s.half_base + (long long)y * nzh + kz0;
+  const int nx = s.grid[0], ny = s.grid[1], nz = s.grid[2];
+  const int kz = t.fixed, y0 = t.first, M = t.count;
+  float2 *h = half + s.half_base + (long long)kz * nx * ny + y0;
   const int ld = nx + 1;  // padded lines (bank-conflict-free transpose)
   for (int idx = threadIdx.x; idx < nx * M; idx += blockDim.x) {
     const int x = idx / M, m = idx - x * M;
-    bufa[m * ld + x] = h[x * stride + m];
+    bufa[m * ld + x] = h[(long long)x * ny + m];
   }
   float2 *r = fft_lines(bufa, bufb, M, nx, ld, pl.axis[0], twiddles + pl.axis[0].tw_base, false);
-  const double volume = sysd[t.sys].volume;
-  const double alpha = sysd[t.sys].alpha;
-  const float factor = (float)(M_PI * M_PI / (alpha * alpha));
-  const float two_pref = (float)(2.0 * ONE_4PI_EPS0 / (2.0 * M_PI * volume));
+  const double weight = (kz == 0 || 2 * kz == nz) ? 1.0 : 2.0;
   const float *modx = moduli + s.moduli_base, *mody = modx + nx, *modz = mody + ny;
-  const int ky = y <= ny / 2 ? y : y - ny;
   double energy = 0.0, virial = 0.0;
   for (int idx = threadIdx.x; idx < nx * M; idx += blockDim.x) {
     const int m = idx / nx, mx = idx - m * nx;
-    const int kz = kz0 + m;
-    const int kx = mx <= nx / 2 ? mx : mx - nx;
-    const int at = m * ld + mx;
-    float2 v = r[at];
-    if (kx == 0 && ky == 0 && kz == 0) {
-      r[at] = make_float2(0.f, 0.f);
-      continue;
-    }
-    const float fx = (float)kx, fy = (float)ky, fz = (float)kz;
-    const float cx = fx * s.recip[0] + fy * s.recip[1] + fz * s.recip[2];
-    const float cy = fx * s.recip[3] + fy * s.recip[4] + fz * s.recip[5];
-    const float cz = fx * s.recip[6] + fy * s.recip[7] + fz * s.recip[8];
-    const float m2 = cx * cx + cy * cy + cz * cz;
-    const float kernel = __expf(-factor * m2) / (m2 * modx[mx] * mody[y] * modz[kz]);
-    if (ENERGY) {
-      const double weight = (kz == 0 || 2 * kz == nz) ? 1.0 : 2.0;
-      const double ek = weight * 0.5 * (double)two_pref * (double)kernel * ((double)v.x * v.x + (double)v.y * v.y);
-      energy += ek;
-      virial += ek * (1.0 + (double)factor * (double)m2);
-    }
-    const float sc = kernel * two_pref;
-    r[at] = make_float2(v.x * sc, v.y * sc);
+    const int my = y0 + m;
+    const ConvolveLine line(s, my <= ny / 2 ? my : my - ny, kz, mody[my] * modz[kz]);
+    line.apply<ENERGY>(r[m * ld + mx], mx <= nx / 2 ? mx : mx - nx, modx[mx], weight, energy, virial);
   }
   float2 *other = (r == bufa) ? bufb : bufa;
   float2 *q = fft_lines(r, other, M, nx, ld, pl.axis[0], twiddles + pl.axis[0].tw_base, true);
   for (int idx = threadIdx.x; idx < nx * M; idx += blockDim.x) {
     const int x = idx / M, m = idx - x * M;
-    h[x * stride + m] = q[m * ld + x];
+    h[(long long)x * ny + m] = q[m * ld + x];
   }
-  if (ENERGY) {
-    energy = warp_sum(energy);
-    virial = warp_sum(virial);
-    if ((threadIdx.x & 31) == 0) {
-      red[0][threadIdx.x >> 5] = energy;
-      red[1][threadIdx.x >> 5] = virial;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double total = 0, total_vir = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        total += red[0][w];
-        total_vir += red[1][w];
+  if (ENERGY) block_energy(energy, virial, e_pme, e_pme_vir, blockIdx.x);
+}
+
+// ------------------------------------------------------------------ two-factor transforms
+// The passes below hold a line of N = R1 * R2 points as R1 rows of R2 (pitch R2 made odd, so
+// that a thread's row and the threads' columns both fall in different shared-memory banks) and
+// transform it in place, one DFT a thread (fft.cuh). Against the Stockham stages they replaced
+// (radix 4, one barrier and one trip through shared memory a stage, the lines copied in and out
+// in passes of their own) each transform is two steps and one barrier, with the first and last
+// step of a pass reading or writing global memory directly. The static inputs (task, twiddles,
+// moduli) are read before a kernel waits for its predecessor.
+__host__ __device__ inline int odd_pitch(int r2) { return r2 | 1; }
+
+constexpr int FFT_PAIRS = FFT_PAIRS_PER_BLOCK;  // pairs of real lines a z block transforms
+
+// z pass, forward (R2C): FFT_PAIRS pairs of real lines, each pair one complex line. The half
+// spectrum is stored plane by plane, half[kz][x * ny + y], so a block's 2 * FFT_PAIRS
+// consecutive lines are one 128-byte run of each plane. All of a thread's 2 R1 loads of the
+// fixed-point grid are in flight together, and the grid is cleared behind them.
+template <int MAXR>
+__global__ void __launch_bounds__(256) k_fft_r2c(const FftZTask *__restrict__ tasks,
+                                                 const float2 *__restrict__ twiddles,
+                                                 unsigned long long *__restrict__ fixed_grid,
+                                                 float2 *__restrict__ half) {
+  extern __shared__ float2 smem[];
+  __shared__ float2 tw[FFT_TWO_MAX];
+  const FftZTask t = tasks[blockIdx.x];
+  const FftTwo &ax = t.z;
+  const int N = ax.n, R1 = ax.r1, R2 = ax.r2, M = t.count, plane = t.plane;
+  const int pitch = odd_pitch(R2), ld = (R1 * pitch) | 1;
+  for (int k = threadIdx.x; k < N; k += blockDim.x) tw[k] = twiddles[ax.tw_base + k];
+  chain_begin();
+  unsigned long long *g = fixed_grid + t.grid_base;
+  with_radix<MAXR>(R1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    for (int it = threadIdx.x; it < M * R2; it += blockDim.x) {
+      const int p = fast_div(it, ax.r2_div), j = it - p * R2;
+      const int l = 2 * (t.first + p);
+      const bool two = l + 1 < plane;
+      unsigned long long *src = g + (long long)l * N + j;
+      unsigned long long a[R], b[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        a[r] = src[r * R2];
+        b[r] = two ? src[N + r * R2] : 0ull;
       }
-      e_pme[blockIdx.x] = total;
-      e_pme_vir[blockIdx.x] = total_vir;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {  // cleared for the next step's spreading
+        src[r * R2] = 0ull;
+        if (two) src[N + r * R2] = 0ull;
+      }
+      float2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = make_float2(from_fixed(a[r]), from_fixed(b[r]));
+      dft<R, false>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) smem[p * ld + r * pitch + j] = v[r];
+    }
+  });
+  __syncthreads();
+  with_radix<MAXR>(R2, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    for (int it = threadIdx.x; it < M * R1; it += blockDim.x) {
+      const int p = fast_div(it, ax.r1_div), k1 = it - p * R1;
+      float2 *line = smem + p * ld + k1 * pitch;
+      float2 v[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) v[j] = cmul(line[j], tw[k1 * j]);
+      dft<R, false>(v);
+#pragma unroll
+      for (int j = 0; j < R; ++j) line[j] = v[j];
+    }
+  });
+  __syncthreads();
+  float2 *h = half + t.half_base;
+  const int nzh = N / 2 + 1;
+  const bool wide = (plane & 1) == 0;  // then a pair's two values are 16-byte aligned in every plane
+  for (int idx = threadIdx.x; idx < FFT_PAIRS * nzh; idx += blockDim.x) {
+    const int p = idx % FFT_PAIRS, k = idx / FFT_PAIRS;
+    if (p >= M) continue;
+    const int l = 2 * (t.first + p), kc = k == 0 ? 0 : N - k;
+    const int q = fast_div(k, ax.r1_div), qc = fast_div(kc, ax.r1_div);
+    const float2 z = smem[p * ld + (k - q * R1) * pitch + q];
+    const float2 zc = smem[p * ld + (kc - qc * R1) * pitch + qc];
+    // A = (Z + conj(Zc))/2, B = -i (Z - conj(Zc))/2
+    const float2 a = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
+    const float2 b = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
+    float2 *out = h + (long long)k * plane + l;
+    if (wide) {
+      *reinterpret_cast<float4 *>(out) = make_float4(a.x, a.y, b.x, b.y);
+    } else {
+      out[0] = a;
+      if (l + 1 < plane) out[1] = b;
     }
   }
 }
 
+// z pass, inverse (C2R), the same shape backwards.
+template <int MAXR>
+__global__ void __launch_bounds__(256) k_fft_c2r(const FftZTask *__restrict__ tasks,
+                                                 const float2 *__restrict__ twiddles,
+                                                 const float2 *__restrict__ half, float *__restrict__ real_grid) {
+  extern __shared__ float2 smem[];
+  __shared__ float2 tw[FFT_TWO_MAX];
+  const FftZTask t = tasks[blockIdx.x];
+  const FftTwo &ax = t.z;
+  const int N = ax.n, R1 = ax.r1, R2 = ax.r2, M = t.count, plane = t.plane;
+  const int pitch = odd_pitch(R2), ld = (R1 * pitch) | 1;
+  const int nzh = N / 2 + 1;
+  for (int k = threadIdx.x; k < N; k += blockDim.x) tw[k] = twiddles[ax.tw_base + k];
+  chain_begin();
+  const float2 *h = half + t.half_base;
+  const bool wide = (plane & 1) == 0;
+  with_radix<MAXR>(R2, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    for (int it = threadIdx.x; it < FFT_PAIRS * R1; it += blockDim.x) {
+      const int p = it % FFT_PAIRS, k1 = it / FFT_PAIRS;
+      if (p >= M) continue;
+      const int l = 2 * (t.first + p);
+      const bool two = l + 1 < plane;
+      float2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int k = k1 + r * R1;
+        const bool mirrored = k >= nzh;
+        const float2 *in = h + (long long)(mirrored ? N - k : k) * plane + l;
+        float2 a, b;
+        if (wide) {
+          const float4 ab = __ldg(reinterpret_cast<const float4 *>(in));
+          a = make_float2(ab.x, ab.y);
+          b = make_float2(ab.z, ab.w);
+        } else {
+          a = __ldg(in);
+          b = two ? __ldg(in + 1) : make_float2(0.f, 0.f);
+        }
+        if (k == 0 || 2 * k == N) a.y = b.y = 0.f;
+        if (mirrored) a.y = -a.y, b.y = -b.y;
+        v[r] = make_float2(a.x - b.y, a.y + b.x);  // A + iB
+      }
+      dft<R, true>(v);
+#pragma unroll
+      for (int j = 0; j < R; ++j) smem[p * ld + k1 * pitch + j] = v[j];
+    }
+  });
+  __syncthreads();
+  float *g = real_grid + t.grid_base;
+  with_radix<MAXR>(R1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    for (int it = threadIdx.x; it < M * R2; it += blockDim.x) {
+      const int p = fast_div(it, ax.r2_div), j = it - p * R2;
+      const int l = 2 * (t.first + p);
+      float2 v[R];
+#pragma unroll
+      for (int k1 = 0; k1 < R; ++k1) {
+        const float2 w = tw[k1 * j];
+        v[k1] = cmul(smem[p * ld + k1 * pitch + j], make_float2(w.x, -w.y));
+      }
+      dft<R, true>(v);
+      float *out = g + (long long)l * N + j;
+#pragma unroll
+      for (int r = 0; r < R; ++r) out[r * R2] = v[r].x;
+      if (l + 1 < plane)
+#pragma unroll
+        for (int r = 0; r < R; ++r) out[N + r * R2] = v[r].y;
+    }
+  });
+}
+
+// ----------------- y and x passes of one kz plane fused: forward y, forward x, the Ewald
+// convolution (and energy), inverse x, inverse y, by a cluster of `cl` blocks a plane (1 for
+// small planes, which a block holds alone). Block r of a cluster owns the x rows
+// [r * rows_per, ...) for the y transforms and the columns [r * cols_per, ...) of the
+// transformed rows for the x transforms and the convolution. Each line is transformed in place
+// (see above) in seven steps:
+//   1 y columns-DFT, from global      2 y rows-DFT            (cluster barrier: rows complete)
+//   3 x columns-DFT, from the owners' rows (distributed shared memory)
+//   4 x rows-DFT, convolution, inverse x rows-DFT, all in registers
+//   5 inverse x columns-DFT, into the owners' rows, once every block has read them (step 3)
+//                                     (cluster barrier: rows complete)
+//   6 inverse y rows-DFT              7 inverse y columns-DFT, to global
+// The convolution needs a column's true ky: column c = k1 * R2 + k2 is ky = k1 + R1 * k2.
+// `threads` of the plan (not the launch's block size, which other systems of a batch may have
+// raised) share the items of each step, so the energy partials' grouping, and with it every bit
+// of the energy, depends on the system alone.
+struct PlaneTables {
+  float2 tw_y[FFT_TWO_MAX], tw_x[FFT_TWO_MAX];
+  float mod_x[FFT_TWO_MAX], mod_y[FFT_TWO_MAX];
+};
+
+template <bool ENERGY, int MAXR>
+__global__ void __launch_bounds__(FFT_PLANE_THREADS)
+    k_fft_planes(const FftPlaneTask *__restrict__ tasks, const DevSys *__restrict__ sys, const float2 *__restrict__ twiddles,
+                 const float *__restrict__ moduli, float2 *__restrict__ half, int cl, int row_stride,
+                 double *__restrict__ e_pme, double *__restrict__ e_pme_vir) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = cl > 1 ? (int)cluster.block_rank() : 0;
+  extern __shared__ float2 smem[];
+  __shared__ PlaneTables tab;
+  const FftPlaneTask t = tasks[blockIdx.x / cl];
+  const FftTwo &ay = t.y, &axx = t.x;
+  const int nx = axx.n, ny = ay.n, kz = t.kz;
+  const int R1y = ay.r1, R2y = ay.r2, R1x = axx.r1, R2x = axx.r2;
+  const int pitch = odd_pitch(R2y), ldy = R1y * pitch;
+  const int rows_per = t.rows_div.d, cols_per = t.cols_div.d;
+  const int x0 = min(nx, rank * rows_per), nr = min(nx, x0 + rows_per) - x0;
+  const int c0 = min(ny, rank * cols_per), nc = min(ny, c0 + cols_per) - c0;
+  const int nt = t.threads, tid = threadIdx.x < nt ? threadIdx.x : INT_MAX;
+  float2 *rows = smem;
+  // the columns' own buffer holds point x of local column c at x * cols_per + c; a block that
+  // owns the whole plane works on the columns in place
+  float2 *cols = cl > 1 ? smem + row_stride : smem;
+  const int cstride = cl > 1 ? cols_per : ldy;
+  float2 *h = half + t.half_base;  // element (x, y) at h[x * ny + y]
+  const float *mod = moduli + t.moduli_base;
+  for (int k = threadIdx.x; k < ny; k += blockDim.x) {
+    tab.tw_y[k] = twiddles[ay.tw_base + k];
+    tab.mod_y[k] = mod[nx + k];
+  }
+  for (int k = threadIdx.x; k < nx; k += blockDim.x) {
+    tab.tw_x[k] = twiddles[axx.tw_base + k];
+    tab.mod_x[k] = mod[k];
+  }
+  const float mod_z = mod[nx + ny + kz];
+  chain_begin();
+  const DevSys &s = sys[t.sys];
+  with_radix<MAXR>(R1y, [&](auto rc) {  // 1
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < nr * R2y; it += nt) {
+      const int row = fast_div(it, ay.r2_div), j = it - row * R2y;
+      const float2 *in = h + (long long)(x0 + row) * ny + j;
+      float2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = in[r * R2y];
+      dft<R, false>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) rows[row * ldy + r * pitch + j] = v[r];
+    }
+  });
+  __syncthreads();
+  with_radix<MAXR>(R2y, [&](auto rc) {  // 2
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < nr * R1y; it += nt) {
+      const int row = fast_div(it, ay.r1_div), k1 = it - row * R1y;
+      float2 *line = rows + row * ldy + k1 * pitch;
+      float2 v[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) v[j] = cmul(line[j], tab.tw_y[k1 * j]);
+      dft<R, false>(v);
+#pragma unroll
+      for (int j = 0; j < R; ++j) line[j] = v[j];
+    }
+  });
+  if (cl > 1) cluster.sync();
+  else __syncthreads();
+  with_radix<MAXR>(R1x, [&](auto rc) {  // 3
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < cols_per * R2x; it += nt) {
+      const int j = fast_div(it, t.cols_div), c = it - j * cols_per;
+      if (c >= nc) continue;  // (the last block of a cluster may own fewer)
+      const int k1y = fast_div(c0 + c, ay.r2_div), at = (c0 + c) + (pitch - R2y) * k1y;  // the column in a row
+      float2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int x = r * R2x + j;
+        const int owner = cl > 1 ? fast_div(x, t.rows_div) : 0;
+        const float2 *src = cl > 1 ? cluster.map_shared_rank(rows, owner) : rows;
+        v[r] = src[(x - owner * rows_per) * ldy + at];
+      }
+      dft<R, false>(v);
+      float2 *col = cols + (cl > 1 ? c : at);
+#pragma unroll
+      for (int r = 0; r < R; ++r) col[(r * R2x + j) * cstride] = v[r];
+    }
+  });
+  if (cl > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");  // this block has read the others' rows
+  __syncthreads();
+  double energy = 0.0, virial = 0.0;
+  const double weight = (kz == 0 || 2 * kz == t.nz) ? 1.0 : 2.0;
+  with_radix<MAXR>(R2x, [&](auto rc) {  // 4
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < cols_per * R1x; it += nt) {
+      const int k1 = fast_div(it, t.cols_div), c = it - k1 * cols_per;
+      if (c >= nc) continue;
+      const int k1y = fast_div(c0 + c, ay.r2_div), k2y = (c0 + c) - k1y * R2y;
+      const int ky = k1y + R1y * k2y;
+      float2 *col = cols + (cl > 1 ? c : k1y * pitch + k2y) + (long long)k1 * R2x * cstride;
+      float2 v[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) v[j] = cmul(col[j * cstride], tab.tw_x[k1 * j]);
+      dft<R, false>(v);
+      const ConvolveLine line(s, ky <= ny / 2 ? ky : ky - ny, kz, tab.mod_y[ky] * mod_z);
+#pragma unroll
+      for (int k2 = 0; k2 < R; ++k2) {
+        const int mx = k1 + R1x * k2;
+        line.apply<ENERGY>(v[k2], mx <= nx / 2 ? mx : mx - nx, tab.mod_x[mx], weight, energy, virial);
+      }
+      dft<R, true>(v);
+#pragma unroll
+      for (int j = 0; j < R; ++j) col[j * cstride] = v[j];
+    }
+  });
+  __syncthreads();
+  if (cl > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // every block has read these rows
+  with_radix<MAXR>(R1x, [&](auto rc) {  // 5
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < cols_per * R2x; it += nt) {
+      const int j = fast_div(it, t.cols_div), c = it - j * cols_per;
+      if (c >= nc) continue;  // (the last block of a cluster may own fewer)
+      const int k1y = fast_div(c0 + c, ay.r2_div), at = (c0 + c) + (pitch - R2y) * k1y;
+      const float2 *col = cols + (cl > 1 ? c : at);
+      float2 v[R];
+#pragma unroll
+      for (int k1 = 0; k1 < R; ++k1) {
+        const float2 w = tab.tw_x[k1 * j];
+        v[k1] = cmul(col[(k1 * R2x + j) * cstride], make_float2(w.x, -w.y));
+      }
+      dft<R, true>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int x = r * R2x + j;
+        const int owner = cl > 1 ? fast_div(x, t.rows_div) : 0;
+        float2 *dst = cl > 1 ? cluster.map_shared_rank(rows, owner) : rows;
+        dst[(x - owner * rows_per) * ldy + at] = v[r];
+      }
+    }
+  });
+  if (cl > 1) cluster.sync();
+  else __syncthreads();
+  with_radix<MAXR>(R2y, [&](auto rc) {  // 6
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < nr * R1y; it += nt) {
+      const int row = fast_div(it, ay.r1_div), k1 = it - row * R1y;
+      float2 *line = rows + row * ldy + k1 * pitch;
+      float2 v[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) v[j] = line[j];
+      dft<R, true>(v);
+#pragma unroll
+      for (int j = 0; j < R; ++j) line[j] = v[j];
+    }
+  });
+  __syncthreads();
+  with_radix<MAXR>(R1y, [&](auto rc) {  // 7
+    constexpr int R = decltype(rc)::value;
+    for (int it = tid; it < nr * R2y; it += nt) {
+      const int row = fast_div(it, ay.r2_div), j = it - row * R2y;
+      float2 v[R];
+#pragma unroll
+      for (int k1 = 0; k1 < R; ++k1) {
+        const float2 w = tab.tw_y[k1 * j];
+        v[k1] = cmul(rows[row * ldy + k1 * pitch + j], make_float2(w.x, -w.y));
+      }
+      dft<R, true>(v);
+      float2 *out = h + (long long)(x0 + row) * ny + j;
+#pragma unroll
+      for (int r = 0; r < R; ++r) out[r * R2y] = v[r];
+    }
+  });
+  if (ENERGY) block_energy(energy, virial, e_pme, e_pme_vir, blockIdx.x);
+}
 // ------------------------------------------------------------------------- gather
-template <int ORDER>
-__global__ void k_gather(const float4 *__restrict__ posq, const int *__restrict__ sys_of_atom,
-                         const DevSys *__restrict__ sys, const float *__restrict__ real_grid,
-                         unsigned long long *__restrict__ force, int n_atoms) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_atoms) return;
-  const float4 p = posq[i];
-  if (p.w == 0.f) return;
-  const DevSys &s = sys[sys_of_atom[i]];
-  float w[3][ORDER], dw[3][ORDER];
-  int base[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float f = p.x * s.recip[d] + p.y * s.recip[3 + d] + p.z * s.recip[6 + d];
-    const float scaled = (f - floorf(f)) * (float)s.grid[d];
-    const float fl = floorf(scaled);
-    base[d] = (int)fl;
-    bspline<ORDER>(scaled - fl, w[d], dw[d]);
-  }
-  const int nx = s.grid[0], ny = s.grid[1], nz = s.grid[2];
-  const float *g = real_grid + s.grid_base;
-  float gu = 0.f, gv = 0.f, gw = 0.f;
-#pragma unroll
-  for (int kx = 0; kx < ORDER; ++kx) {
-    const int ix = wrap_index(base[0] + kx - ORDER + 1, nx);
-#pragma unroll
-    for (int ky = 0; ky < ORDER; ++ky) {
-      const int iy = wrap_index(base[1] + ky - ORDER + 1, ny);
-      const float *rowp = g + ((long long)ix * ny + iy) * nz;
-      const float wxy = w[0][kx] * w[1][ky], dxy = dw[0][kx] * w[1][ky], wdy = w[0][kx] * dw[1][ky];
-#pragma unroll
-      for (int kz = 0; kz < ORDER; ++kz) {
-        const int iz = wrap_index(base[2] + kz - ORDER + 1, nz);
-        const float v = __ldg(rowp + iz);
-        gu = fmaf(dxy * w[2][kz], v, gu);
-        gv = fmaf(wdy * w[2][kz], v, gv);
-        gw = fmaf(wxy * dw[2][kz], v, gw);
-      }
-    }
-  }
-  const float su = gu * (float)nx * p.w, sv = gv * (float)ny * p.w, sw = gw * (float)nz * p.w;
-  add_fixed(force + i, -(su * s.recip[0] + sv * s.recip[1] + sw * s.recip[2]));
-  add_fixed(force + n_atoms + i, -(su * s.recip[3] + sv * s.recip[4] + sw * s.recip[5]));
-  add_fixed(force + 2 * (long long)n_atoms + i, -(su * s.recip[6] + sv * s.recip[7] + sw * s.recip[8]));
-}
-
 // Force gather with four threads per atom (atoms in cell order, for locality of the grid
 // reads): thread q sums the x-planes kx = q, q + 4 (< ORDER), the four partial gradients are
 // combined with shuffles, and the first thread adds the force. One thread per atom leaves
@@ -533,7 +808,11 @@ static void launch_forward_zy(const LaunchCtx &c, cudaStream_t stream, bool all 
   // boundary. Chained after the spreading it was slower on one B200 at 64^3 (the seven
   // reciprocal kernels 0.067 against 0.049 ms, the 23,558-atom step 0.1394 against 0.1358 ms)
   // and no faster at 32^3 or 100^3. It still lets the next pass be scheduled early.
-  k_fft_z_r2c<<<c.n_tasks_z, 256, 0, stream>>>(c.tasks_z, c.sys, c.fft_plans, c.twiddles, c.fixed_grid, c.half);
+  if (c.n_tasks_z2 > 0)
+    (c.fft_large ? k_fft_r2c<RADIX_ALL> : k_fft_r2c<RADIX_SMALL>)<<<c.n_tasks_z2, c.z2_threads, c.z2_smem * sizeof(float2), stream>>>(
+        c.tasks_z2, c.twiddles, c.fixed_grid, c.half);
+  if (c.n_tasks_z > 0)
+    k_fft_z_r2c<<<c.n_tasks_z, 256, 0, stream>>>(c.tasks_z, c.sys, c.fft_plans, c.twiddles, c.fixed_grid, c.half);
   const FftTask *ty = all ? c.tasks_y_all : c.tasks_y;
   const int n = all ? c.n_tasks_y_all : c.n_tasks_y;
   if (n > 0) launch_kernel(c.chain_pme, k_fft_y, n, 256, 0, stream, ty, c.sys, c.fft_plans, c.twiddles, c.half, 0);
@@ -543,267 +822,66 @@ static void launch_inverse_yz(const LaunchCtx &c, cudaStream_t stream, bool all 
   const FftTask *ty = all ? c.tasks_y_all : c.tasks_y;
   const int n = all ? c.n_tasks_y_all : c.n_tasks_y;
   if (n > 0) launch_kernel(c.chain_pme, k_fft_y, n, 256, 0, stream, ty, c.sys, c.fft_plans, c.twiddles, c.half, 1);
-  launch_kernel(c.chain_pme, k_fft_z_c2r, c.n_tasks_z, 256, 0, stream, c.tasks_z, c.sys, c.fft_plans, c.twiddles, c.half,
-                c.real_grid);
-}
-
-// A plane pass's per-axis tables in shared memory: the y and x twiddles and B-spline moduli,
-// copied once when the plane is loaded (in the same round trip as the plane) instead of before
-// each of the four transforms. Planes on these passes have nx, ny <= TW_CACHE.
-struct PlaneTables {
-  float2 tw_y[TW_CACHE], tw_x[TW_CACHE];
-  float mod_x[TW_CACHE], mod_y[TW_CACHE];
-};
-
-// Fill the tables (visible after the barrier that opens the first transform stage); returns
-// the z moduli, read from global memory (one value a plane).
-__device__ __forceinline__ const float *stage_plane_tables(PlaneTables &tab, const FftPlan &pl,
-                                                           const float2 *__restrict__ twiddles,
-                                                           const float *__restrict__ mod, int nx, int ny) {
-  for (int k = threadIdx.x; k < ny; k += blockDim.x) {
-    tab.tw_y[k] = twiddles[pl.axis[1].tw_base + k];
-    tab.mod_y[k] = mod[nx + k];
-  }
-  for (int k = threadIdx.x; k < nx; k += blockDim.x) {
-    tab.tw_x[k] = twiddles[pl.axis[0].tw_base + k];
-    tab.mod_x[k] = mod[k];
-  }
-  return mod + nx + ny;
-}
-
-// The Ewald convolution of one half-spectrum point (x index mx, y index my, plane kz) in place,
-// with its energy and virial terms added when ENERGY: the per-point arithmetic of
-// k_fft_x_convolve, shared by the fused plane passes.
-template <bool ENERGY>
-__device__ __forceinline__ void convolve_point(float2 &v, int mx, int my, int kz, int nx, int ny, int nz,
-                                               const DevSys &s, const float *modx, const float *mody,
-                                               const float *modz, float factor, float two_pref,
-                                               double &energy, double &virial) {
-  const int kx = mx <= nx / 2 ? mx : mx - nx;
-  const int ky = my <= ny / 2 ? my : my - ny;
-  if (kx == 0 && ky == 0 && kz == 0) {
-    v = make_float2(0.f, 0.f);
-    return;
-  }
-  const float fx = (float)kx, fy = (float)ky, fz = (float)kz;
-  const float cx = fx * s.recip[0] + fy * s.recip[1] + fz * s.recip[2];
-  const float cy = fx * s.recip[3] + fy * s.recip[4] + fz * s.recip[5];
-  const float cz = fx * s.recip[6] + fy * s.recip[7] + fz * s.recip[8];
-  const float m2 = cx * cx + cy * cy + cz * cz;
-  const float kernel = __expf(-factor * m2) / (m2 * modx[mx] * mody[my] * modz[kz]);
-  if (ENERGY) {
-    const double weight = (kz == 0 || 2 * kz == nz) ? 1.0 : 2.0;
-    const double ek = weight * 0.5 * (double)two_pref * (double)kernel * ((double)v.x * v.x + (double)v.y * v.y);
-    energy += ek;
-    virial += ek * (1.0 + (double)factor * (double)m2);
-  }
-  const float sc = kernel * two_pref;
-  v = make_float2(v.x * sc, v.y * sc);
-}
-
-// Block sum of a thread's energy and virial terms, written by thread 0 to e[slot], ev[slot].
-__device__ __forceinline__ void block_energy(double energy, double virial, double *e, double *ev, int slot) {
-  __shared__ double red[2][256 / 32];
-  energy = warp_sum(energy);
-  virial = warp_sum(virial);
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = energy;
-    red[1][threadIdx.x >> 5] = virial;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double total = 0, total_vir = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      total += red[0][w];
-      total_vir += red[1][w];
-    }
-    e[slot] = total;
-    ev[slot] = total_vir;
-  }
-}
-
-// ----------------- y and x passes of one kz plane fused: forward y, forward x, the Ewald
-// convolution (and energy), inverse x, inverse y, with the whole plane in shared memory. One
-// block per (system, kz) plane of the half spectrum, for systems with small planes (see
-// fft_plane_split): three launches and two trips of the half spectrum through L2 become
-// one. The energy partial is the plane's, so a system's partials are grouped the same way in a
-// batch as alone.
-template <bool ENERGY>
-__global__ void __launch_bounds__(256) k_fft_plane(const FftTask *__restrict__ tasks,
-                                                   const DevSys *__restrict__ sys,
-                                                   const DevSysD *__restrict__ sysd,
-                                                   const FftPlan *__restrict__ plans,
-                                                   const float2 *__restrict__ twiddles,
-                                                   const float *__restrict__ moduli,
-                                                   float2 *__restrict__ half, int plane_stride,
-                                                   double *__restrict__ e_pme, double *__restrict__ e_pme_vir) {
-  chain_begin();
-  extern __shared__ float2 plane_smem[];
-  __shared__ PlaneTables tab;
-  float2 *bufa = plane_smem, *bufb = plane_smem + plane_stride;
-  const FftTask t = tasks[blockIdx.x];
-  const DevSys &s = sys[t.sys];
-  const FftPlan &pl = plans[t.sys];
-  const int nx = s.grid[0], ny = s.grid[1], nz = s.grid[2], nzh = nz / 2 + 1;
-  const int kz = t.fixed;
-  const int ldy = ny + 1, ldx = nx + 1;  // padded lines (bank-conflict-free transposes)
-  float2 *h = half + s.half_base + kz;  // element (x, y) at h[(x * ny + y) * nzh]
-  for (int idx = threadIdx.x; idx < nx * ny; idx += blockDim.x) {
-    const int x = fast_div(idx, pl.axis[1].n_div), y = idx - x * ny;
-    bufa[x * ldy + y] = h[(long long)idx * nzh];
-  }
-  const float *modz = stage_plane_tables(tab, pl, twiddles, moduli + s.moduli_base, nx, ny);
-  // forward y: nx lines of ny
-  float2 *r = fft_stages(bufa, bufb, nx, ny, ldy, pl.axis[1], tab.tw_y, false);
-  float2 *o = (r == bufa) ? bufb : bufa;
-  for (int idx = threadIdx.x; idx < nx * ny; idx += blockDim.x) {
-    const int x = fast_div(idx, pl.axis[1].n_div), y = idx - x * ny;
-    o[y * ldx + x] = r[x * ldy + y];
-  }
-  // forward x: ny lines of nx
-  r = fft_stages(o, r, ny, nx, ldx, pl.axis[0], tab.tw_x, false);
-  const double volume = sysd[t.sys].volume;
-  const double alpha = sysd[t.sys].alpha;
-  const float factor = (float)(M_PI * M_PI / (alpha * alpha));
-  const float two_pref = (float)(2.0 * ONE_4PI_EPS0 / (2.0 * M_PI * volume));
-  double energy = 0.0, virial = 0.0;
-  for (int idx = threadIdx.x; idx < nx * ny; idx += blockDim.x) {
-    const int y = fast_div(idx, pl.axis[0].n_div), mx = idx - y * nx;
-    convolve_point<ENERGY>(r[y * ldx + mx], mx, y, kz, nx, ny, nz, s, tab.mod_x, tab.mod_y, modz, factor,
-                           two_pref, energy, virial);
-  }
-  // inverse x
-  o = (r == bufa) ? bufb : bufa;
-  r = fft_stages(r, o, ny, nx, ldx, pl.axis[0], tab.tw_x, true);
-  o = (r == bufa) ? bufb : bufa;
-  for (int idx = threadIdx.x; idx < nx * ny; idx += blockDim.x) {
-    const int x = fast_div(idx, pl.axis[1].n_div), y = idx - x * ny;
-    o[x * ldy + y] = r[y * ldx + x];
-  }
-  // inverse y
-  r = fft_stages(o, r, nx, ny, ldy, pl.axis[1], tab.tw_y, true);
-  for (int idx = threadIdx.x; idx < nx * ny; idx += blockDim.x) {
-    const int x = fast_div(idx, pl.axis[1].n_div), y = idx - x * ny;
-    h[(long long)idx * nzh] = r[x * ldy + y];
-  }
-  if (ENERGY) block_energy(energy, virial, e_pme, e_pme_vir, blockIdx.x);
-}
-
-// The same fused pass for larger planes, shared by a thread-block cluster of PLANE_CLUSTER
-// blocks so that a plane is not one block's serial chain. Block r of a cluster owns the x rows
-// [r * rows_per, ...) for the y transforms and the y columns [r * cols_per, ...) for the x
-// transforms and the convolution; between them each block gathers its lines from the other
-// blocks' shared memory (distributed shared memory), with three cluster barriers: after the
-// forward y pass (rows complete), after the inverse x pass (columns complete, and every block
-// done reading the rows), and after the gather back (every block done reading the columns, so
-// none exits while another still reads it). Every line goes through the same transform as in
-// k_fft_plane; the energy partials are one per block of the cluster.
-template <bool ENERGY>
-__global__ void __cluster_dims__(PLANE_CLUSTER, 1, 1) __launch_bounds__(256)
-    k_fft_plane_cluster(const FftTask *__restrict__ tasks, const DevSys *__restrict__ sys,
-                        const DevSysD *__restrict__ sysd, const FftPlan *__restrict__ plans,
-                        const float2 *__restrict__ twiddles, const float *__restrict__ moduli,
-                        float2 *__restrict__ half, int row_stride, int col_stride,
-                        double *__restrict__ e_pme, double *__restrict__ e_pme_vir) {
-  chain_begin();
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  extern __shared__ float2 plane_smem[];
-  __shared__ PlaneTables tab;
-  float2 *ra = plane_smem, *rb = ra + row_stride, *ca = rb + row_stride, *cb = ca + col_stride;
-  const FftTask t = tasks[blockIdx.x / PLANE_CLUSTER];
-  const DevSys &s = sys[t.sys];
-  const FftPlan &pl = plans[t.sys];
-  const int nx = s.grid[0], ny = s.grid[1], nz = s.grid[2], nzh = nz / 2 + 1;
-  const int kz = t.fixed;
-  const int ldy = ny + 1, ldx = nx + 1;
-  const int rows_per = (nx + PLANE_CLUSTER - 1) / PLANE_CLUSTER, cols_per = (ny + PLANE_CLUSTER - 1) / PLANE_CLUSTER;
-  const int x0 = min(nx, rank * rows_per), nr = min(nx, x0 + rows_per) - x0;
-  const int y0 = min(ny, rank * cols_per), nc = min(ny, y0 + cols_per) - y0;
-  float2 *h = half + s.half_base + kz;  // element (x, y) at h[(x * ny + y) * nzh]
-  for (int idx = threadIdx.x; idx < nr * ny; idx += blockDim.x) {
-    const int xl = fast_div(idx, pl.axis[1].n_div), y = idx - xl * ny;
-    ra[xl * ldy + y] = h[((long long)(x0 + xl) * ny + y) * nzh];
-  }
-  const float *modz = stage_plane_tables(tab, pl, twiddles, moduli + s.moduli_base, nx, ny);
-  // forward y over this block's rows; every block runs the same stages, so the result sits
-  // at the same offset in each block's shared memory
-  const float2 *rows = fft_stages(ra, rb, nr, ny, ldy, pl.axis[1], tab.tw_y, false);
-  cluster.sync();
-  for (int idx = threadIdx.x; idx < nc * nx; idx += blockDim.x) {
-    const int yl = fast_div(idx, pl.axis[0].n_div), x = idx - yl * nx;
-    const int owner = x / rows_per;
-    const float2 *src = cluster.map_shared_rank(rows, owner);
-    ca[yl * ldx + x] = src[(x - owner * rows_per) * ldy + y0 + yl];
-  }
-  // forward x over this block's columns, the convolution, inverse x
-  float2 *c = fft_stages(ca, cb, nc, nx, ldx, pl.axis[0], tab.tw_x, false);
-  const double volume = sysd[t.sys].volume;
-  const double alpha = sysd[t.sys].alpha;
-  const float factor = (float)(M_PI * M_PI / (alpha * alpha));
-  const float two_pref = (float)(2.0 * ONE_4PI_EPS0 / (2.0 * M_PI * volume));
-  double energy = 0.0, virial = 0.0;
-  for (int idx = threadIdx.x; idx < nc * nx; idx += blockDim.x) {
-    const int yl = fast_div(idx, pl.axis[0].n_div), mx = idx - yl * nx;
-    convolve_point<ENERGY>(c[yl * ldx + mx], mx, y0 + yl, kz, nx, ny, nz, s, tab.mod_x, tab.mod_y, modz, factor,
-                           two_pref, energy, virial);
-  }
-  const float2 *cols = fft_stages(c, c == ca ? cb : ca, nc, nx, ldx, pl.axis[0], tab.tw_x, true);
-  cluster.sync();
-  for (int idx = threadIdx.x; idx < nr * ny; idx += blockDim.x) {
-    const int xl = fast_div(idx, pl.axis[1].n_div), y = idx - xl * ny;
-    const int owner = y / cols_per;
-    const float2 *src = cluster.map_shared_rank(cols, owner);
-    ra[xl * ldy + y] = src[(y - owner * cols_per) * ldx + x0 + xl];
-  }
-  cluster.sync();
-  // inverse y over this block's rows
-  const float2 *r = fft_stages(ra, rb, nr, ny, ldy, pl.axis[1], tab.tw_y, true);
-  for (int idx = threadIdx.x; idx < nr * ny; idx += blockDim.x) {
-    const int xl = fast_div(idx, pl.axis[1].n_div), y = idx - xl * ny;
-    h[((long long)(x0 + xl) * ny + y) * nzh] = r[xl * ldy + y];
-  }
-  if (ENERGY) block_energy(energy, virial, e_pme, e_pme_vir, blockIdx.x);
+  if (c.n_tasks_z2 > 0)
+    launch_kernel(c.chain_pme, c.fft_large ? k_fft_c2r<RADIX_ALL> : k_fft_c2r<RADIX_SMALL>, c.n_tasks_z2, c.z2_threads, c.z2_smem * sizeof(float2), stream, c.tasks_z2,
+                  c.twiddles, c.half, c.real_grid);
+  if (c.n_tasks_z > 0)
+    launch_kernel(c.chain_pme, k_fft_z_c2r, c.n_tasks_z, 256, 0, stream, c.tasks_z, c.sys, c.fft_plans, c.twiddles,
+                  c.half, c.real_grid);
 }
 
 // Planes of at most this many points go to one block each. A block's plane is one serial
-// chain, so larger grids run faster shared by a cluster: measured on one B200 (the seven
-// reciprocal kernels) one block a plane is faster than the separate passes at 32^3 (0.037
-// against 0.041 ms) and for 64 grids of 22^3-50^3 together (0.30 against 0.34 ms), slower at
-// 64^3 (0.071 against 0.056 ms) and 100^3 (0.194 against 0.152 ms). A cluster a plane for
-// those 64 small grids too was slower again (0.375 ms): their 1,150 planes fill the GPU already.
+// chain, so larger grids run faster shared by a cluster; a batch's small grids fill the GPU with
+// one block a plane already (the line between the two was measured with the Stockham passes: one
+// block a plane at 64^3 0.071 ms for the reciprocal kernels against 0.056 ms in a cluster, and a
+// cluster a plane for 64 grids of 22^3-50^3 0.375 against 0.30 ms).
 constexpr long long PLANE_SINGLE_MAX = 52 * 52;
 
+// A block's shared buffers for a plane of a system: its rows, and (in a cluster) its columns.
 void fft_plane_buffers(int nx, int ny, int split, int *rows, int *cols) {
-  if (split == 1) {
-    *rows = *cols = std::max(nx * (ny + 1), ny * (nx + 1));
-    return;
-  }
-  *rows = (nx + split - 1) / split * (ny + 1);
-  *cols = (ny + split - 1) / split * (nx + 1);
+  int r1 = 1, r2 = 1;
+  fft_two_factors(ny, &r1, &r2);
+  *rows = (nx + split - 1) / split * r1 * (r2 | 1);
+  *cols = split > 1 ? (ny + split - 1) / split * nx : 0;
+}
+
+// Threads that share a plane block's steps: one a DFT of the widest step, within the block limit.
+int fft_plane_threads(int nx, int ny, int split) {
+  int r1x = 1, r2x = 1, r1y = 1, r2y = 1;
+  fft_two_factors(nx, &r1x, &r2x);
+  fft_two_factors(ny, &r1y, &r2y);
+  const int items = std::max((nx + split - 1) / split * std::max(r1y, r2y), (ny + split - 1) / split * std::max(r1x, r2x));
+  // (a cluster's blocks: two rounds when there are more than 256, so that two blocks share an SM)
+  const int threads = split > 1 && items > 256 ? (items + 1) / 2 : items;
+  return std::min(FFT_PLANE_THREADS, std::max(64, (threads + 31) / 32 * 32));
 }
 
 // The rule depends on the system alone, so a system takes the same pass in a batch as alone.
-// A cluster block's row and column buffers are each held to half the limit, so that the
-// largest rows and the largest columns of different systems in one launch still fit together.
+// Planes up to PLANE_SINGLE_MAX points: one block; larger ones a cluster while a block's quarter
+// of the rows and of the columns stays within PLANE_QUARTER_MAX points (128 x 128 and a little
+// beyond; the largest rows and the largest columns of different systems in one launch still fit
+// a block's shared memory together); larger planes and axes without two factors: separate passes.
+constexpr int PLANE_QUARTER_MAX = 6400;
+static bool plane_axis(int n) {
+  int r1, r2, rest = n;
+  for (int p : {2, 3, 5})
+    while (rest > 0 && rest % p == 0) rest /= p;
+  // (an axis that is not 5-smooth is on no grid: the rule answers for its size alone)
+  return n >= 1 && n <= FFT_TWO_MAX && (rest != 1 || fft_two_factors(n, &r1, &r2));
+}
 int fft_plane_split(int nx, int ny) {
-  int rows, cols;
-  fft_plane_buffers(nx, ny, 1, &rows, &cols);
-  if (nx > TW_CACHE || ny > TW_CACHE) return 0;
-  if ((long long)nx * ny <= PLANE_SINGLE_MAX && 2LL * rows * (long long)sizeof(float2) <= FFT_PLANE_SMEM_MAX) return 1;
+  if (!plane_axis(nx) || !plane_axis(ny)) return 0;
+  if ((long long)nx * ny <= PLANE_SINGLE_MAX) return 1;
   if (nx < PLANE_CLUSTER || ny < PLANE_CLUSTER) return 0;
-  fft_plane_buffers(nx, ny, PLANE_CLUSTER, &rows, &cols);
-  const long long half_limit = FFT_PLANE_SMEM_MAX / 2;
-  if (2LL * rows * (long long)sizeof(float2) <= half_limit && 2LL * cols * (long long)sizeof(float2) <= half_limit)
-    return PLANE_CLUSTER;
-  return 0;
+  const int rows_per = (nx + PLANE_CLUSTER - 1) / PLANE_CLUSTER, cols_per = (ny + PLANE_CLUSTER - 1) / PLANE_CLUSTER;
+  return rows_per * (ny + 1) <= PLANE_QUARTER_MAX && cols_per * (nx + 1) <= PLANE_QUARTER_MAX ? PLANE_CLUSTER : 0;
 }
 
 // The largest dynamic shared memory the plane kernels may take, set once per device before any
 // launch (and never lowered, so engines with different grids cannot undercut each other).
 cudaError_t fft_plane_prepare() {
-  const void *fns[4] = {(const void *)k_fft_plane<true>, (const void *)k_fft_plane<false>,
-                        (const void *)k_fft_plane_cluster<true>, (const void *)k_fft_plane_cluster<false>};
+  const void *fns[4] = {(const void *)k_fft_planes<true, RADIX_SMALL>, (const void *)k_fft_planes<false, RADIX_SMALL>,
+                        (const void *)k_fft_planes<true, RADIX_ALL>, (const void *)k_fft_planes<false, RADIX_ALL>};
   for (const void *f : fns) {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FFT_PLANE_SMEM_MAX);
     if (e != cudaSuccess) return e;
@@ -814,25 +892,34 @@ cudaError_t fft_plane_prepare() {
 static void launch_planes(const LaunchCtx &c, bool energy, cudaStream_t stream) {
   // partials after the x tasks': the planes' one each, then the clusters' PLANE_CLUSTER each
   double *e = c.e_pme + c.n_tasks_x, *ev = c.e_pme_vir + c.n_tasks_x;
-  if (c.n_tasks_plane > 0) {
-    const size_t smem = 2 * (size_t)c.plane_stride * sizeof(float2);
-    launch_kernel(c.chain_pme, energy ? k_fft_plane<true> : k_fft_plane<false>, c.n_tasks_plane, 256, smem, stream,
-                   c.tasks_plane, c.sys, c.sysd, c.fft_plans, c.twiddles, c.moduli, c.half, c.plane_stride, e, ev);
-  }
-  if (c.n_tasks_cluster > 0) {
-    e += c.n_tasks_plane;
-    ev += c.n_tasks_plane;
-    const size_t smem = 2 * ((size_t)c.cluster_rows + c.cluster_cols) * sizeof(float2);
-    launch_kernel(c.chain_pme, energy ? k_fft_plane_cluster<true> : k_fft_plane_cluster<false>,
-                  c.n_tasks_cluster * PLANE_CLUSTER,
-                   256, smem, stream, c.tasks_cluster, c.sys, c.sysd, c.fft_plans, c.twiddles, c.moduli, c.half,
-                   c.cluster_rows, c.cluster_cols, e, ev);
-  }
+  auto launch = [&](int cl, const FftPlaneTask *tasks, int n, int threads, int rows, int cols) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n * cl);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = ((size_t)rows + cols) * sizeof(float2);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cl;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = c.chain_pme ? 2 : 1;
+    auto kernel = c.fft_large ? (energy ? k_fft_planes<true, RADIX_ALL> : k_fft_planes<false, RADIX_ALL>)
+                              : (energy ? k_fft_planes<true, RADIX_SMALL> : k_fft_planes<false, RADIX_SMALL>);
+    (void)cudaLaunchKernelEx(&cfg, kernel, tasks, (const DevSys *)c.sys, c.twiddles, c.moduli, c.half, cl, rows, e, ev);
+  };
+  if (c.n_tasks_plane > 0) launch(1, c.tasks_plane, c.n_tasks_plane, c.plane_threads, c.plane_stride, 0);
+  e += c.n_tasks_plane;
+  ev += c.n_tasks_plane;
+  if (c.n_tasks_cluster > 0)
+    launch(PLANE_CLUSTER, c.tasks_cluster, c.n_tasks_cluster, c.cluster_threads, c.cluster_rows, c.cluster_cols);
 }
 
 int pme_launches(const LaunchCtx &c) {
   if (!c.pme_on) return 0;
-  return 4 + (c.n_tasks_plane > 0 ? 1 : 0) + (c.n_tasks_cluster > 0 ? 1 : 0) + (c.n_tasks_x > 0 ? 3 : 0);
+  return 2 + 2 * ((c.n_tasks_z > 0 ? 1 : 0) + (c.n_tasks_z2 > 0 ? 1 : 0)) + (c.n_tasks_plane > 0 ? 1 : 0) + (c.n_tasks_cluster > 0 ? 1 : 0) + (c.n_tasks_x > 0 ? 3 : 0);
 }
 
 // Everything up to the convolved real grid: spreading, forward transform, convolution (and
@@ -842,7 +929,7 @@ static void launch_transform_convolve(const LaunchCtx &c, bool energy, cudaStrea
   launch_planes(c, energy, stream);
   if (c.n_tasks_x > 0)
     launch_kernel(c.chain_pme, energy ? k_fft_x_convolve<true> : k_fft_x_convolve<false>, c.n_tasks_x, 256, 0, stream,
-                   c.tasks_x, c.sys, c.sysd, c.fft_plans, c.twiddles, c.moduli, c.half, c.e_pme, c.e_pme_vir);
+                   c.tasks_x, c.sys, c.fft_plans, c.twiddles, c.moduli, c.half, c.e_pme, c.e_pme_vir);
   launch_inverse_yz(c, stream);
 }
 
@@ -873,19 +960,17 @@ __global__ void k_fft_x_plain(const FftTask *__restrict__ tasks, const DevSys *_
   const FftTask t = tasks[blockIdx.x];
   const DevSys &s = sys[t.sys];
   const FftPlan &pl = plans[t.sys];
-  const int nx = s.grid[0], ny = s.grid[1], nzh = s.grid[2] / 2 + 1;
-  const int y = t.fixed, kz0 = t.first, M = t.count;
-  const long long stride = (long long)ny * nzh;
-  float2 *h = half + s.half_base + (long long)y * nzh + kz0;
+  const int nx = s.grid[0], ny = s.grid[1], M = t.count;
+  float2 *h = half + s.half_base + (long long)t.fixed * nx * ny + t.first;
   const int ld = nx + 1;
   for (int idx = threadIdx.x; idx < nx * M; idx += blockDim.x) {
     const int x = idx / M, m = idx - x * M;
-    bufa[m * ld + x] = h[x * stride + m];
+    bufa[m * ld + x] = h[(long long)x * ny + m];
   }
   float2 *r = fft_lines(bufa, bufb, M, nx, ld, pl.axis[0], twiddles + pl.axis[0].tw_base, inverse != 0);
   for (int idx = threadIdx.x; idx < nx * M; idx += blockDim.x) {
     const int x = idx / M, m = idx - x * M;
-    h[x * stride + m] = r[m * ld + x];
+    h[(long long)x * ny + m] = r[m * ld + x];
   }
 }
 

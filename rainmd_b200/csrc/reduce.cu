@@ -94,6 +94,8 @@ __device__ void set_box(DevSys &s, DevSysD &d, const double *b) {
   s.inv_diag[1] = (float)(1.0 / by);
   s.inv_diag[2] = (float)(1.0 / cz);
   d.volume = fabs(ax * by * cz);
+  s.pme_factor = (float)(M_PI * M_PI / (d.alpha * d.alpha));
+  s.pme_pref = (float)(2.0 * ONE_4PI_EPS0 / (2.0 * M_PI * d.volume));
   // Cells at least the list cutoff wide (cells.js:101-171), never more than allocated.
   const double w[3] = {fabs(ax), fabs(by), fabs(cz)};
   for (int k = 0; k < 3; ++k) {
