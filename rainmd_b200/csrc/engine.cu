@@ -260,6 +260,9 @@ struct Engine {
   DevArray<int> free_atoms, cl_atom_start, cl_atoms, cl_con_start;
   DevArray<int2> cl_con_pair;
   DevArray<float> cl_con_dist;
+  DevArray<int4> shaped_atoms;
+  DevArray<float4> shaped_dist;
+  int shaped_end[4] = {0, 0, 0, 0};
   DevArray<int3> settle_atoms;
   DevArray<DevSettle> settle_param;
   int n_free = 0, n_clusters = 0, n_settle = 0;
@@ -722,6 +725,8 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   e_term_vir.zero();
 
   // ---- constraint clusters (buildConstraintClusters, clusters.js:20-57) and SETTLE waters
+  std::vector<int4> h_shaped[4];
+  std::vector<float4> h_shaped_d[4];
   std::vector<int> h_free, h_cl_as, h_cl_atoms, h_cl_cs;
   std::vector<int2> h_pairs;
   std::vector<float> h_dist;
@@ -813,6 +818,28 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
                                          std::to_string(members.size()) +
                                          " constraints exceeds the per-thread solver limit (8 atoms, 12 "
                                          "constraints); use HBonds constraints");
+      // clusters of a fixed shape: the triangle, or one atom bound to one, two or three others
+      // (which of the two ends of a constraint comes first must match too)
+      const int nc = (int)members.size(), na = (int)atoms.size();
+      auto joins = [&](int k, int p, int q) {
+        return r.constraint_atoms[2 * members[k]] == atoms[p] && r.constraint_atoms[2 * members[k] + 1] == atoms[q];
+      };
+      int shape = -1;
+      if (nc == 3 && na == 3 && joins(0, 0, 1) && joins(1, 0, 2) && joins(2, 1, 2)) shape = 0;
+      else if (nc <= 3 && na == nc + 1) {
+        shape = nc;
+        for (int k = 0; k < nc; ++k)
+          if (!joins(k, 0, k + 1)) shape = -1;
+      }
+      if (shape >= 0) {
+        int4 w = make_int4(base + atoms[0], base + atoms[1], na > 2 ? base + atoms[2] : 0, na > 3 ? base + atoms[3] : 0);
+        float4 d = make_float4((float)r.constraint_distance[members[0]], nc > 1 ? (float)r.constraint_distance[members[1]] : 0.f,
+                               nc > 2 ? (float)r.constraint_distance[members[2]] : 0.f, 0.f);
+        h_shaped[shape].push_back(w);
+        h_shaped_d[shape].push_back(d);
+        h.n_clusters++;
+        continue;
+      }
       for (int a : atoms) h_cl_atoms.push_back(base + a);
       h_cl_as.push_back((int)h_cl_atoms.size());
       for (int k : members) {
@@ -828,10 +855,22 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
     for (int a = 0; a < h.n; ++a)
       if (!in_cluster[a]) h_free.push_back(base + a);
   }
-  // units in order: free atoms, SHAKE clusters, SETTLE waters
+  // units in order: free atoms, SHAKE clusters (any shape, then the fixed ones), SETTLE waters
   n_free = (int)h_free.size();
   n_clusters = (int)h_cl_as.size() - 1;
   n_settle = (int)h_settle.size();
+  {
+    std::vector<int4> w;
+    std::vector<float4> d;
+    for (int k = 0; k < 4; ++k) {
+      w.insert(w.end(), h_shaped[k].begin(), h_shaped[k].end());
+      d.insert(d.end(), h_shaped_d[k].begin(), h_shaped_d[k].end());
+      shaped_end[k] = (int)w.size();
+    }
+    if (w.empty()) w.push_back(make_int4(0, 0, 0, 0)), d.push_back(make_float4(0.f, 0.f, 0.f, 0.f));
+    shaped_atoms.upload(w);
+    shaped_dist.upload(d);
+  }
   if (h_free.empty()) h_free.push_back(0);
   if (h_cl_atoms.empty()) h_cl_atoms.push_back(0);
   if (h_pairs.empty()) {
@@ -1387,7 +1426,10 @@ IntegrateArgs Engine::iargs(int step_offset) const {
   a.n_free = n_free;
   a.n_clusters = n_clusters;
   a.n_settle = n_settle;
-  a.n_units = n_free + n_clusters + n_settle;
+  a.n_units = n_free + n_clusters + shaped_end[3] + n_settle;
+  a.shaped_atoms = shaped_atoms.p;
+  a.shaped_dist = shaped_dist.p;
+  for (int k = 0; k < 4; ++k) a.shaped_end[k] = shaped_end[k];
   a.n_atoms = N;
   a.n_systems = S;
   a.free_atoms = free_atoms.p;

@@ -85,6 +85,10 @@ struct IntegrateArgs {
   const int *cl_atom_start, *cl_atoms, *cl_con_start;
   const int2 *cl_con_pair;
   const float *cl_con_dist;
+  // clusters of a fixed shape (integrate.cu ClusterShape), shape s up to shaped_end[s]
+  const int4 *shaped_atoms;
+  const float4 *shaped_dist;
+  int shaped_end[4];
   const int3 *settle_atoms;
   const DevSettle *settle_param;
   const int *sys_of_atom;
