@@ -256,6 +256,7 @@ struct Engine {
   DevArray<int> diag;
   DevArray<double> energies, saved_energies, baro, seg_out, fixed_scales;
   DevArray<Segment> segments;
+  DevArray<int> term_first;
   int n_segments = 0;
   DevArray<int> free_atoms, cl_atom_start, cl_atoms, cl_con_start;
   DevArray<int2> cl_con_pair;
@@ -1241,32 +1242,44 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   // ---- energy segments
   {
     std::vector<Segment> seg;
+    std::vector<int> first;
+    struct Range {
+      int term;
+      const double *data;
+      long long start, end;
+    };
     auto recip_begin = [&](int s) { return recip_lo[s]; };
     auto recip_end = [&](int s) { return recip_hi[s]; };
     for (int s = 0; s < S; ++s) {
       const HostSystem &h = hs[s];
+      std::vector<Range> ranges;
       const long long a0 = h.atom_start, a1 = h.atom_start + h.n;
-      seg.push_back(Segment{s, E_BOND, e_term.p, bstart[s], bstart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_ANGLE, e_term.p, n_bonds + astart[s], n_bonds + astart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_TORSION, e_term.p, n_bonds + n_angles + tstart[s],
-                            n_bonds + n_angles + tstart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_RESTRAINT, e_term.p, n_bonds + n_angles + n_tors + rstart[s],
-                            n_bonds + n_angles + n_tors + rstart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_LJ, e_lj.p, a0, a1, nullptr});
-      seg.push_back(Segment{s, E_COUL_DIRECT, e_coul.p, a0, a1, nullptr});
-      seg.push_back(Segment{s, E_RECIP, e_pme.p, recip_begin(s), recip_end(s), nullptr});
-      seg.push_back(Segment{s, E_VIR_SR, e_vir.p, a0, a1, nullptr});
-      seg.push_back(Segment{s, E_VIR_SR, e_term_vir.p, bstart[s], bstart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_VIR_SR, e_term_vir.p, n_bonds + astart[s], n_bonds + astart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_VIR_SR, e_term_vir.p, n_bonds + n_angles + tstart[s],
-                            n_bonds + n_angles + tstart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_VIR_SR, e_term_vir.p, n_bonds + n_angles + n_tors + rstart[s],
-                            n_bonds + n_angles + n_tors + rstart[s + 1], nullptr});
-      seg.push_back(Segment{s, E_VIR_MOL, mol_vir.p, mol_base[s], mol_base[s + 1], nullptr});
-      seg.push_back(Segment{s, E_VIR_REC, e_pme_vir.p, recip_begin(s), recip_end(s), nullptr});
-      seg.push_back(Segment{s, E_KINETIC, ke_post.p, a0, a1, nullptr});
-      seg.push_back(Segment{s, E_KINETIC_EARLY, ke_early.p, a0, a1, nullptr});
+      ranges.push_back(Range{E_BOND, e_term.p, bstart[s], bstart[s + 1]});
+      ranges.push_back(Range{E_ANGLE, e_term.p, n_bonds + astart[s], n_bonds + astart[s + 1]});
+      ranges.push_back(Range{E_TORSION, e_term.p, n_bonds + n_angles + tstart[s], n_bonds + n_angles + tstart[s + 1]});
+      ranges.push_back(Range{E_RESTRAINT, e_term.p, n_bonds + n_angles + n_tors + rstart[s], n_bonds + n_angles + n_tors + rstart[s + 1]});
+      ranges.push_back(Range{E_LJ, e_lj.p, a0, a1});
+      ranges.push_back(Range{E_COUL_DIRECT, e_coul.p, a0, a1});
+      ranges.push_back(Range{E_RECIP, e_pme.p, recip_begin(s), recip_end(s)});
+      ranges.push_back(Range{E_VIR_SR, e_vir.p, a0, a1});
+      ranges.push_back(Range{E_VIR_SR, e_term_vir.p, bstart[s], bstart[s + 1]});
+      ranges.push_back(Range{E_VIR_SR, e_term_vir.p, n_bonds + astart[s], n_bonds + astart[s + 1]});
+      ranges.push_back(Range{E_VIR_SR, e_term_vir.p, n_bonds + n_angles + tstart[s], n_bonds + n_angles + tstart[s + 1]});
+      ranges.push_back(Range{E_VIR_SR, e_term_vir.p, n_bonds + n_angles + n_tors + rstart[s], n_bonds + n_angles + n_tors + rstart[s + 1]});
+      ranges.push_back(Range{E_VIR_MOL, mol_vir.p, mol_base[s], mol_base[s + 1]});
+      ranges.push_back(Range{E_VIR_REC, e_pme_vir.p, recip_begin(s), recip_end(s)});
+      ranges.push_back(Range{E_KINETIC, ke_post.p, a0, a1});
+      ranges.push_back(Range{E_KINETIC_EARLY, ke_early.p, a0, a1});
+      for (int term = 0; term < N_ENERGY; ++term) {
+        first.push_back((int)seg.size());
+        for (const Range &r : ranges)
+          for (long long k = r.start; r.term == term && k < r.end; k += SEGMENT_CHUNK)
+            seg.push_back(Segment{r.data, k, std::min(r.end, k + SEGMENT_CHUNK)});
+      }
     }
+    first.push_back((int)seg.size());
+    term_first.upload(first);
+    if (seg.empty()) seg.push_back(Segment{e_lj.p, 0, 0});
     n_segments = (int)seg.size();
     segments.upload(seg);
     seg_out.alloc(n_segments);
@@ -1579,7 +1592,7 @@ void Engine::record_forces(int rebuild, bool energy) {
   recorded += nonbonded_launches(c, energy) + (n_bonds + n_angles + n_tors + n_rest > 0 ? 1 : 0) + pme_launches(c);
   if (energy) {
     launch_molecular_virial(c, stream);
-    launch_energy_reduce(segments.p, n_segments, seg_out.p, energies.p, sysd.p, S, stream);
+    launch_energy_reduce(segments.p, n_segments, term_first.p, seg_out.p, energies.p, sysd.p, S, stream);
     recorded += 3;
   }
 }

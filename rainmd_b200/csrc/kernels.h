@@ -247,8 +247,8 @@ void launch_integrate(const IntegrateArgs &a, int mode, cudaStream_t stream);
 void launch_draws(uint32_t seed, uint32_t atom0, int count, uint32_t step, float *uniforms, float *normals,
                   cudaStream_t stream);
 
-// Energy segments reduced per system (reduce.cu). Each segment is [start, end) of one
-// per-item FP64 array; the result lands in energies[sys * N_ENERGY + term].
+// Energy terms reduced per system (reduce.cu), in chunks [start, end) of per-item FP64 arrays; the
+// results land in energies[sys * N_ENERGY + term].
 enum EnergyTerm {
   E_BOND = 0, E_ANGLE, E_TORSION, E_LJ, E_COUL_DIRECT, E_RECIP, E_RESTRAINT, E_KINETIC,
   E_KINETIC_EARLY, E_SELF, E_NET, E_DISPERSION, E_POTENTIAL,
@@ -259,12 +259,13 @@ enum EnergyTerm {
   E_VIR_SR, E_VIR_REC, E_VIR_MOL, E_DUDLNV, N_ENERGY
 };
 struct Segment {
-  int sys, term;
   const double *data;
-  long long start, end;
-  const double *data2;  // optional second array summed over the same range (LJ: nonbonded)
+  long long start, end;  // at most SEGMENT_CHUNK items
 };
-void launch_energy_reduce(const Segment *segments, int n_segments, double *seg_out,
+constexpr int SEGMENT_CHUNK = 4096;
+// term_first[s * N_ENERGY + t]: the first chunk of system s's term t (chunks are ordered by system,
+// then term; one entry past the last)
+void launch_energy_reduce(const Segment *segments, int n_segments, const int *term_first, double *seg_out,
                           double *energies, const DevSysD *sysd, int n_systems, cudaStream_t stream);
 
 // Barostat and utility kernels (reduce.cu).

@@ -1,9 +1,9 @@
 // Deterministic FP64 energy reductions and the on-device Monte Carlo barostat.
 //
 // Energies: every energy-producing kernel writes per-item FP64 contributions (per atom,
-// per bonded term, per PME block); one block per segment sums its range in a fixed order,
-// and one thread per system adds the segments in a fixed order and the volume-dependent
-// constants: Ewald self and net-charge terms (cpu/forces/pme.js:270-286) and the LJ
+// per bonded term, per PME block); one block per SEGMENT_CHUNK items sums its run in a fixed
+// order, and one block per system adds each term's chunks in a fixed order and the
+// volume-dependent constants: Ewald self and net-charge terms (cpu/forces/pme.js:270-286) and the LJ
 // dispersion correction (shared/dispersion.js:76-82). Same bits every run.
 //
 // Barostat: the reference's attemptVolumeChange (webgpu/simulation.js:995-1070) does two
@@ -18,13 +18,13 @@
 
 namespace rmd {
 
+// One block a chunk of at most SEGMENT_CHUNK items (a block a term took 257 us at 250,000 atoms, a
+// thousand dependent rounds of loads; 6 us split), cut from the term's first item on, so a
+// system's sums are grouped the same way in a batch as alone.
 __global__ void k_segment_sum(const Segment *__restrict__ segs, double *__restrict__ out) {
   const Segment sg = segs[blockIdx.x];
   double acc = 0.0;
-  for (long long k = sg.start + threadIdx.x; k < sg.end; k += blockDim.x) {
-    acc += sg.data[k];
-    if (sg.data2) acc += sg.data2[k];
-  }
+  for (long long k = sg.start + threadIdx.x; k < sg.end; k += blockDim.x) acc += sg.data[k];
   __shared__ double red[32];
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -36,15 +36,22 @@ __global__ void k_segment_sum(const Segment *__restrict__ segs, double *__restri
   }
 }
 
-__global__ void k_energy_finalize(const Segment *__restrict__ segs, int n_segments,
-                                  const double *__restrict__ seg_out, double *__restrict__ energies,
-                                  const DevSysD *__restrict__ sysd, int n_systems) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_systems) return;
-  double e[N_ENERGY];
-  for (int k = 0; k < N_ENERGY; ++k) e[k] = 0.0;
-  for (int k = 0; k < n_segments; ++k)
-    if (segs[k].sys == s) e[segs[k].term] += seg_out[k];
+// One block a system: a warp sums the chunks of each term (term_first: where the chunks of each
+// system and term begin), then one thread adds the constants. (One thread a system walking every
+// segment of the batch took 96 us for 24 systems; 5 us this way.)
+__global__ void k_energy_finalize(const int *__restrict__ term_first, const double *__restrict__ seg_out,
+                                  double *__restrict__ energies, const DevSysD *__restrict__ sysd) {
+  const int s = blockIdx.x;
+  __shared__ double e[N_ENERGY];
+  for (int t = threadIdx.x >> 5; t < N_ENERGY; t += blockDim.x >> 5) {
+    const int end = term_first[s * N_ENERGY + t + 1];
+    double acc = 0.0;
+    for (int k = term_first[s * N_ENERGY + t] + (threadIdx.x & 31); k < end; k += 32) acc += seg_out[k];
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) e[t] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   const DevSysD d = sysd[s];
   const double sqrt_pi = 1.7724538509055160273;
   if (d.alpha > 0) {
@@ -68,11 +75,10 @@ __global__ void k_energy_finalize(const Segment *__restrict__ segs, int n_segmen
   for (int k = 0; k < N_ENERGY; ++k) energies[s * N_ENERGY + k] = e[k];
 }
 
-void launch_energy_reduce(const Segment *segments, int n_segments, double *seg_out,
+void launch_energy_reduce(const Segment *segments, int n_segments, const int *term_first, double *seg_out,
                           double *energies, const DevSysD *sysd, int n_systems, cudaStream_t stream) {
   if (n_segments > 0) k_segment_sum<<<n_segments, 256, 0, stream>>>(segments, seg_out);
-  k_energy_finalize<<<(n_systems + 63) / 64, 64, 0, stream>>>(segments, n_segments, seg_out,
-                                                              energies, sysd, n_systems);
+  k_energy_finalize<<<n_systems, 256, 0, stream>>>(term_first, seg_out, energies, sysd);
 }
 
 // ------------------------------------------------------------------------ box helpers
@@ -191,18 +197,21 @@ __global__ void k_baro_propose(BaroArgs a) {
   set_box(a.sys[s], d, nb);
 }
 
-// One warp per molecule: mass-weighted centroid (FP64 accumulation), then shift every
+// WIDTH lanes (1 or 32) per molecule: mass-weighted centroid (FP64 accumulation), then shift every
 // atom of the molecule by (s - 1) * centroid; the old positions and forces are saved.
-__global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double *__restrict__ fixed_scales) {
-  const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (m >= n_molecules) return;
-  const int begin = a.mol_start[m], end = a.mol_start[m + 1];
+template <int WIDTH>
+__device__ __forceinline__ double lanes_sum(double v) {
+  return WIDTH == 1 ? v : warp_sum(v);
+}
+template <int WIDTH>
+__device__ __forceinline__ void centroid_scale(const BaroArgs &a, const double *__restrict__ fixed_scales, int begin,
+                                               int end, int lane) {
   const int s = a.sys_of_atom[a.mol_atoms[begin]];
   const double ls = fixed_scales ? fixed_scales[s] : a.baro[(long long)s * N_BARO + B_LSCALE];
   // Save positions and forces of this molecule's atoms (restored if the move is rejected), and
   // for a move on the current lists their wrap shifts and displacement origins.
   const bool keep = a.keep_lists && !fixed_scales;
-  for (int k = begin + lane; k < end; k += 32) {
+  for (int k = begin + lane; k < end; k += WIDTH) {
     const int i = a.mol_atoms[k];
     a.saved_posq[i] = a.posq[i];
     a.saved_force[i] = a.force[i];
@@ -215,7 +224,7 @@ __global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double 
   }
   if (ls == 1.0) return;
   double cx = 0, cy = 0, cz = 0, mt = 0;
-  for (int k = begin + lane; k < end; k += 32) {
+  for (int k = begin + lane; k < end; k += WIDTH) {
     const int i = a.mol_atoms[k];
     const float4 p = a.posq[i];
     const double mm = a.masses[i];
@@ -224,21 +233,21 @@ __global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double 
     cz += mm * p.z;
     mt += mm;
   }
-  cx = warp_sum(cx);
-  cy = warp_sum(cy);
-  cz = warp_sum(cz);
-  mt = warp_sum(mt);
+  cx = lanes_sum<WIDTH>(cx);
+  cy = lanes_sum<WIDTH>(cy);
+  cz = lanes_sum<WIDTH>(cz);
+  mt = lanes_sum<WIDTH>(mt);
   if (!(mt > 0)) {  // massless molecule: plain mean (barostat.js:47-58)
     cx = cy = cz = 0;
-    for (int k = begin + lane; k < end; k += 32) {
+    for (int k = begin + lane; k < end; k += WIDTH) {
       const float4 p = a.posq[a.mol_atoms[k]];
       cx += p.x;
       cy += p.y;
       cz += p.z;
     }
-    cx = warp_sum(cx);
-    cy = warp_sum(cy);
-    cz = warp_sum(cz);
+    cx = lanes_sum<WIDTH>(cx);
+    cy = lanes_sum<WIDTH>(cy);
+    cz = lanes_sum<WIDTH>(cz);
     mt = (double)(end - begin);
   }
   cx /= mt;
@@ -246,7 +255,7 @@ __global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double 
   cz /= mt;
   const double f = ls - 1.0;
   float spread = 0.f;  // the molecule's largest atom-centroid distance
-  for (int k = begin + lane; k < end; k += 32) {
+  for (int k = begin + lane; k < end; k += WIDTH) {
     const int i = a.mol_atoms[k];
     float4 p = a.posq[i];
     if (keep) {
@@ -271,8 +280,21 @@ __global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double 
     }
   }
   if (keep) {
-    spread = warp_max(spread);
+    if (WIDTH > 1) spread = warp_max(spread);
     if (lane == 0) atomic_max_nonneg(&a.spread_bits[s], spread);
+  }
+}
+
+// A molecule of up to SMALL_MOLECULE atoms is one thread's; the larger ones among a warp's 32 are
+// taken by the whole warp in turn (a warp for every molecule left 29 of 32 lanes idle on water).
+constexpr int SMALL_MOLECULE = 8;
+__global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double *__restrict__ fixed_scales) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int begin = m < n_molecules ? a.mol_start[m] : 0, end = m < n_molecules ? a.mol_start[m + 1] : 0;
+  if (end > begin && end - begin <= SMALL_MOLECULE) centroid_scale<1>(a, fixed_scales, begin, end, 0);
+  for (unsigned large = __ballot_sync(0xffffffffu, end - begin > SMALL_MOLECULE); large; large &= large - 1u) {
+    const int from = __ffs(large) - 1;
+    centroid_scale<32>(a, fixed_scales, __shfl_sync(0xffffffffu, begin, from), __shfl_sync(0xffffffffu, end, from), lane);
   }
 }
 
@@ -385,11 +407,11 @@ void launch_baro_propose(const BaroArgs &a, cudaStream_t stream) {
 }
 void launch_baro_scale(const BaroArgs &a, cudaStream_t stream) {
   const int tb = 128;
-  k_baro_centroid_scale<<<(a.n_molecules * 32 + tb - 1) / tb, tb, 0, stream>>>(a, a.n_molecules, nullptr);
+  k_baro_centroid_scale<<<(a.n_molecules + tb - 1) / tb, tb, 0, stream>>>(a, a.n_molecules, nullptr);
 }
 void launch_scale_fixed(const BaroArgs &a, const double *scales, cudaStream_t stream) {
   const int tb = 128;
-  k_baro_centroid_scale<<<(a.n_molecules * 32 + tb - 1) / tb, tb, 0, stream>>>(a, a.n_molecules, scales);
+  k_baro_centroid_scale<<<(a.n_molecules + tb - 1) / tb, tb, 0, stream>>>(a, a.n_molecules, scales);
 }
 void launch_baro_allow(const BaroArgs &a, cudaStream_t stream) {
   k_baro_allow<<<(a.n_systems + 63) / 64, 64, 0, stream>>>(a);
