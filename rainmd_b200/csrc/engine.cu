@@ -215,7 +215,7 @@ struct Engine {
   // group-pair rows (pair_list 0 and 2): rows, lengths, first order position and atoms per group
   // slot; per slot its partner record and order position; per-atom integer energy sums
   int pair_list = 1;
-  DevArray<int> gnbr, gnbr_count, gfirst, gsize, order_pos;
+  DevArray<int> gnbr, gnbr_count, gfirst, gsize, group_cell;
   DevArray<float4> group_box;
   // volume moves evaluated on the current lists (reduce.cu k_baro_centroid_scale, k_baro_allow)
   DevArray<float4> saved_wrap, saved_origin;
@@ -990,8 +990,6 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   sorted_type.zero();
   slot_info.alloc(N);
   slot_info.zero();
-  order_pos.alloc(N);
-  order_pos.zero();
   e_acc.alloc(3 * (size_t)N);
   e_acc.zero();
   rank.alloc(N);
@@ -1303,7 +1301,7 @@ void Engine::allocate_neighbours() {
   nbr_count.zero();
   gnbr.alloc(std::max<long long>(1, group_total));
   gnbr.zero();
-  for (auto *a : {&gnbr_count, &gfirst, &gsize}) {
+  for (auto *a : {&gnbr_count, &gfirst, &gsize, &group_cell}) {
     a->alloc(std::max(1, n_groups_total));
     a->zero();
   }
@@ -1358,8 +1356,8 @@ LaunchCtx Engine::ctx() const {
   c.gfirst = gfirst.p;
   c.gsize = gsize.p;
   c.slot_info = slot_info.p;
-  c.order_pos = order_pos.p;
   c.group_box = group_box.p;
+  c.group_cell = group_cell.p;
   c.e_acc = e_acc.p;
   c.origin = origin.p;
   c.spos = spos.p;
@@ -2755,20 +2753,19 @@ rmd_status rmd_debug_group_rows(rmd_sim *sim, int32_t s, int32_t *groups, int32_
     if (groups) *groups = n;
     if (capacity) *capacity = cap;
     if (!atoms && !counts && !partners) return;
-    std::vector<int> size(n), start(n), cnt(n), order(h.n), orig(h.n), raw((size_t)n * cap);
+    std::vector<int> size(n), start(n), cnt(n), orig(h.n), raw((size_t)n * cap);
     CUDA_OK(cudaMemcpy(size.data(), e.gsize.p + first, sizeof(int) * n, cudaMemcpyDeviceToHost));
     CUDA_OK(cudaMemcpy(start.data(), e.gfirst.p + first, sizeof(int) * n, cudaMemcpyDeviceToHost));
     CUDA_OK(cudaMemcpy(cnt.data(), e.gnbr_count.p + first, sizeof(int) * n, cudaMemcpyDeviceToHost));
-    CUDA_OK(cudaMemcpy(order.data(), e.group_order.p + h.atom_start, sizeof(int) * h.n, cudaMemcpyDeviceToHost));
     CUDA_OK(cudaMemcpy(orig.data(), e.sorted_orig.p + h.atom_start, sizeof(int) * h.n, cudaMemcpyDeviceToHost));
     CUDA_OK(cudaMemcpy(raw.data(), e.gnbr.p + ds.gnbr_base, sizeof(int) * raw.size(), cudaMemcpyDeviceToHost));
-    // slots and order positions are global: map both back to the system's own atom indices
+    // slots are global, a group's consecutive: mapped back to the system's own atom indices
     auto atom_of_slot = [&](int slot) { return orig[slot - h.atom_start] - h.atom_start; };
     for (int q = 0; q < n; ++q) {
       for (int a = 0; a < rmd::GROUP_ATOMS; ++a)
         if (atoms)
           atoms[q * rmd::GROUP_ATOMS + a] =
-              a < size[q] ? atom_of_slot(order[start[q] + a - h.atom_start]) : -1;
+              a < size[q] ? atom_of_slot(start[q] + a) : -1;
       if (counts) counts[q] = size[q] > 0 ? cnt[q] : 0;
       for (int k = 0; k < cap; ++k) {
         const bool used = size[q] > 0 && k < cnt[q];

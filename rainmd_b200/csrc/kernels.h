@@ -136,7 +136,7 @@ struct LaunchCtx {
   int *gnbr, *gnbr_count;  // group-pair rows and their lengths, per group slot
   int *gfirst, *gsize;     // per group slot: its first position in group_order, its atoms (0: unused)
   int2 *slot_info;         // per slot: LJ type, original index
-  int *order_pos;          // per slot: its position in group_order
+  int *group_cell;         // per group slot: its cell
   float4 *group_box;       // per group slot: bounding box lo, hi of its atoms' wrapped positions
   unsigned long long *e_acc;  // per-atom integer energy sums of the group-pair kernel (3 N)
   bool force_cleared;  // the force array was zeroed since the last evaluation (launch_nonbonded skips its clear)

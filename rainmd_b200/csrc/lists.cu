@@ -29,11 +29,12 @@ struct LaunchCtxView {
   int *sorted_orig, *sorted_type, *rank;
   int *group_order;
   int2 *slot_info;  // per slot: LJ type, original index (the group-pair kernel's partner record)
-  int *order_pos;   // per slot: its position in group_order
   // group-pair rows only (else null): per 4-atom group slot its bounding box (lo, hi) of wrapped
-  // positions, and the cell scan's first group per cell
+  // positions, and the cell scan's first group per cell. The slots are then numbered in search
+  // order, so that a group's atoms are consecutive slots; otherwise by ascending index in the cell.
   float4 *group_box;
   const int *cell_gstart;
+  int *group_cell;  // per 4-atom group slot: its cell
 };
 
 __global__ void k_cells_assign(const float4 *__restrict__ posq, const int *__restrict__ sys_of_atom,
@@ -158,16 +159,11 @@ __device__ __forceinline__ int hilbert_key(int x, int y, int z) {
   return h;
 }
 
-// Write slot g's cell-ordered record for atom j: its position shifted into the box by
-// whole box vectors (the shift is kept per atom so the integrator can apply it every step).
-// Returns the atom's sub-cell key: the Hilbert index of its position on a 4x4x4 grid inside
-// its cell (the order in which the neighbour search groups a cell's atoms).
-__device__ __forceinline__ int place_sorted(const LaunchCtxView &v, const DevSys &s, int g, int j,
-                                            const int cc[3]) {
-  const float4 p = v.posq[j];
-  // floor of the same exact-rounding fractional coordinate the cell assignment used, so the
-  // wrapped copy lies in (the closure of) the cell the atom was counted in
-  float fl[3];
+// Atom j's sub-cell key, the Hilbert index of its position on a 4x4x4 grid inside its cell (the
+// order in which the neighbour search groups a cell's atoms), and in `fl` the whole box vectors
+// to take off its position: floor of the same exact-rounding fractional coordinate the cell
+// assignment used, so the wrapped copy lies in (the closure of) the cell the atom was counted in.
+__device__ __forceinline__ int sub_cell_key(const float4 p, const DevSys &s, const int cc[3], float (&fl)[3]) {
   int sub[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -176,6 +172,17 @@ __device__ __forceinline__ int place_sorted(const LaunchCtxView &v, const DevSys
     const float inside = (f - fl[d]) * (float)s.cell_counts[d] - (float)cc[d];
     sub[d] = min(3, max(0, (int)(inside * 4.f)));
   }
+  return hilbert_key(sub[0], sub[1], sub[2]);
+}
+
+// Write slot g's cell-ordered record for atom j: its position shifted into the box by
+// whole box vectors (the shift is kept per atom so the integrator can apply it every step).
+// Returns the atom's sub-cell key.
+__device__ __forceinline__ int place_sorted(const LaunchCtxView &v, const DevSys &s, int g, int j,
+                                            const int cc[3]) {
+  const float4 p = v.posq[j];
+  float fl[3];
+  const int key = sub_cell_key(p, s, cc, fl);
   const float wx = fl[0] * s.box[0] + fl[1] * s.box[3] + fl[2] * s.box[6];
   const float wy = fl[0] * s.box[1] + fl[1] * s.box[4] + fl[2] * s.box[7];
   const float wz = fl[0] * s.box[2] + fl[1] * s.box[5] + fl[2] * s.box[8];
@@ -185,12 +192,13 @@ __device__ __forceinline__ int place_sorted(const LaunchCtxView &v, const DevSys
   v.sorted_type[g] = v.atom_type[j];
   v.slot_info[g] = make_int2(v.atom_type[j], j);
   v.rank[j] = g;
-  return hilbert_key(sub[0], sub[1], sub[2]);
+  return key;
 }
 
 // One block per allocated cell: rank-sort the cell's slice ascending, zero the cursor, write
-// the cell-ordered records of its atoms, and order the cell's slots by sub-cell key (ties by
-// slot) into group_order, so that 32 consecutive entries there are spatially compact.
+// the cell-ordered records of its atoms, and order the cell's atoms by sub-cell key (ties by
+// index), so that consecutive ones are spatially compact: into the slots themselves with
+// group-pair rows, else into group_order.
 __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__restrict__ sys,
                              const int *__restrict__ cell_start, int *__restrict__ cell_cursor,
                              int *__restrict__ cell_atoms, LaunchCtxView v, const int *__restrict__ only) {
@@ -211,6 +219,8 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
   constexpr int SMEM = 2048;
   __shared__ int keys[SMEM];
   __shared__ int sub_keys[SMEM];
+  __shared__ int sorted[SMEM];
+  const bool by_group = v.group_box != nullptr;
   if (n <= SMEM) {
     for (int k = threadIdx.x; k < n; k += blockDim.x) keys[k] = slice[k];
     __syncthreads();
@@ -218,14 +228,24 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
       int key = keys[k], rank = 0;
       for (int m = 0; m < n; ++m) rank += keys[m] < key;
       slice[rank] = key;
-      sub_keys[rank] = (place_sorted(v, s, gbase + rank, key, cc) << 11) | rank;
+      if (by_group) {
+        float fl[3];
+        sorted[rank] = key;
+        sub_keys[rank] = (sub_cell_key(v.posq[key], s, cc, fl) << 11) | rank;
+      } else {
+        sub_keys[rank] = (place_sorted(v, s, gbase + rank, key, cc) << 11) | rank;
+      }
     }
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       int key = sub_keys[k], rank = 0;
       for (int m = 0; m < n; ++m) rank += sub_keys[m] < key;
-      v.group_order[gbase + rank] = gbase + k;
-      v.order_pos[gbase + k] = gbase + rank;
+      if (by_group) {
+        place_sorted(v, s, gbase + rank, sorted[k], cc);
+        v.group_order[gbase + k] = gbase + k;
+      } else {
+        v.group_order[gbase + rank] = gbase + k;
+      }
     }
   } else {
     // Oversized cell (only in pathological inputs): serial insertion sort by one thread;
@@ -244,7 +264,6 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       place_sorted(v, s, gbase + k, slice[k], cc);
       v.group_order[gbase + k] = gbase + k;
-      v.order_pos[gbase + k] = gbase + k;
     }
   }
   if (v.group_box) {  // the bounding box of each 4-atom group of this cell, for the search's cull
@@ -253,10 +272,11 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
     for (int k = threadIdx.x; 4 * k < n; k += blockDim.x) {
       float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
       for (int a = 4 * k; a < min(n, 4 * k + 4); ++a) {
-        const float4 p = v.spos[v.group_order[gbase + a]];
+        const float4 p = v.spos[gbase + a];
         lo = make_float4(fminf(lo.x, p.x), fminf(lo.y, p.y), fminf(lo.z, p.z), 0.f);
         hi = make_float4(fmaxf(hi.x, p.x), fmaxf(hi.y, p.y), fmaxf(hi.z, p.z), 0.f);
       }
+      v.group_cell[first_group + k] = c;
       v.group_box[2 * (first_group + k)] = lo;
       v.group_box[2 * (first_group + k) + 1] = hi;
     }
@@ -275,6 +295,9 @@ __device__ __forceinline__ bool is_excluded(const int *__restrict__ start, const
   return false;
 }
 
+// Group slots from which a warp builds a row alone, and from which four warps do instead of eight.
+constexpr int GROUP_ROW_WARP_GROUPS = 148 * 64 * 2;
+constexpr int GROUP_ROW_BLOCK_GROUPS = 148 * 8;
 constexpr int NBR_WARPS = 4;        // groups per block when one warp searches for a group
 constexpr int NBR_SPLIT = 3;        // warps per group in the split search (one stencil x-slab each)
 constexpr int NBR_SPLIT_STAGE = 2048;  // hits a split warp stages in shared memory (G atoms together)
@@ -313,7 +336,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
                  const int *__restrict__ cell_gstart, const int *__restrict__ group_order,
                  const int *__restrict__ excl_start, const int *__restrict__ excl_partners,
                  const float4 *__restrict__ spos, const int *__restrict__ sorted_orig,
-                 int *__restrict__ nbr, int *__restrict__ nbr_count, int *__restrict__ required,
+                 const int *__restrict__ cell_atoms, const int *__restrict__ rank, int *__restrict__ nbr, int *__restrict__ nbr_count, int *__restrict__ required,
                  float4 *__restrict__ origin, int n_groups, const int *__restrict__ only) {
   constexpr int J = 32 / G;
   constexpr int WARPS = SPLIT == 1 ? NBR_WARPS : SPLIT;
@@ -432,10 +455,11 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
           const int begin = s.atom_start + cell_start[s.cell_start_base + cell];
           const int end = s.atom_start + cell_start[s.cell_start_base + cell + 1];
           for (int b = begin; b < end; b += 32) {
-            const int g = b + lane;
+            int g = b + lane;
             bool keep = g < end;
             float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
             if (keep) {
+              if (cell_atoms) g = rank[cell_atoms[g]];  // slots in search order: the g-th atom by index
               pj = spos[g];
               if (stencil_shift) {  // drop candidates beyond the list cutoff from the bounding box
                 const float c[3] = {pj.x, pj.y, pj.z};
@@ -566,13 +590,13 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
 
 // ---------------------------------------------------------------- group-pair rows
 // One WARP per search group of GROUP_ATOMS atoms (the groups of k_neighbours<4, 1>): the
-// group's row lists every partner atom that lies within the list cutoff of the group's
-// bounding box through some lattice image, once per such image, and only if the pair belongs
-// to this group: the partner comes later in search order (order_pos beyond the group), or it
+// group's row lists every partner atom that lies within the list cutoff of one of the group's
+// atoms through some lattice image, once per such image, and only if the pair belongs
+// to this group: the partner comes later in search order (its slot is beyond the group's), or it
 // is one of the group's own atoms, when the entry's mask keeps only the pairs seen from the
 // group's earlier atoms. Mask bits also mark the excluded pairs (cells.js:191-227) and the
 // atoms past the end of a short group. Every pair within the list cutoff of its two atoms is
-// therefore listed exactly once over all rows (the bounding box contains the atom), and an
+// therefore listed exactly once over all rows (the test's margin covers its f32 rounding), and an
 // atom is never paired with its own image.
 //
 // With at least three cells on every axis the stencil reaches each cell through one lattice
@@ -580,27 +604,39 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
 // lattice images -1, 0, +1 of the axes with fewer than three cells, so that every image of a
 // partner within the list cutoff is found.
 //
-// A block of GROUP_ROW_WARPS warps builds one group's row: the stencil's cells are dealt out to
-// the warps in turn, and each warp appends its survivors behind a shared-memory counter, so the
-// row is several short serial walks instead of one long one. The order of a row's entries then
-// depends on the warps' timing; its contents do not, and neither does any force (every pair's
-// fixed-point force is added whatever the order).
-constexpr int GROUP_ROW_WARPS = 4;
-__global__ void __launch_bounds__(32 * GROUP_ROW_WARPS)
+// A block of WARPS warps builds one group's row. The visits (a stencil cell through an image) are
+// decided 32 at a time, a lane each: a cell before the group's own holds only atoms earlier in
+// search order, whose groups list those pairs, and in a rectangular box a cell whose image lies
+// beyond the list cutoff of the group's box is skipped (a 2 x 2 x 2-cell box has 216 visits, of
+// which some 40 are near). The lanes also read their visits' group and slot ranges, so that the walk
+// over the needed ones starts from registers. The needed visits are dealt to the warps in turn and
+// each warp appends its survivors behind a shared-memory counter, so the row is several short serial
+// walks instead of one long one; with enough groups to fill the GPU a warp a row does the same with
+// less work. The order of a row's entries then depends on the warps' timing; its contents do not, and
+// neither does any force (every pair's fixed-point force is added whatever the order). The rebuild's
+// kernels, before and with this form: 250,000 atoms (a warp a row) 814 -> 512 us, 99,999 353 -> 238, a
+// batch of 24 systems 417 -> 218, 23,558 (four warps) 107 -> 101, 2,854 and 1,190 (eight, most visits
+// dropped) 92 -> 61 and 68 -> 40.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS == 1 ? 128 : 32 * WARPS, WARPS == 8 ? 4 : 8)
     k_group_rows(const float4 *__restrict__ posq, const int *__restrict__ group_sys,
                  const DevSys *__restrict__ sys, const int *__restrict__ cell_start,
-                 const int *__restrict__ cell_gstart, const int *__restrict__ group_order,
+                 const int *__restrict__ cell_gstart, const int *__restrict__ group_cell,
                  const int *__restrict__ excl_start, const int *__restrict__ excl_partners,
                  const float4 *__restrict__ spos, const int2 *__restrict__ slot_info,
                  const float4 *__restrict__ group_box, int *__restrict__ gnbr, int *__restrict__ gnbr_count,
                  int *__restrict__ gfirst, int *__restrict__ gsize, int *__restrict__ required,
                  float4 *__restrict__ origin, int n_groups, const int *__restrict__ only) {
   constexpr int G = GROUP_ATOMS;
-  __shared__ int row_count;
-  __shared__ int survivors[GROUP_ROW_WARPS][32];
-  const int warp = blockIdx.x;  // the group slot (every exit before the barriers is the block's)
-  const int wib = threadIdx.x >> 5;
+  constexpr int BLOCK_WARPS = WARPS == 1 ? 4 : WARPS;  // a warp a row: four rows a block
+  constexpr int ROWS = BLOCK_WARPS / WARPS;
+  __shared__ int row_count[ROWS];
+  __shared__ int survivors[BLOCK_WARPS][32];
+  __shared__ float4 group_near[ROWS][G];
+  __shared__ int4 excluded[ROWS][G];
+  const int wib = threadIdx.x >> 5, part = wib % WARPS, rib = wib / WARPS;
   const int lane = threadIdx.x & 31;
+  const int warp = blockIdx.x * ROWS + rib;  // the group slot (with WARPS > 1 every exit before the barriers is the block's)
   if (warp >= n_groups) return;
   const int sidx = group_sys[warp];
   if (only && !only[sidx]) return;  // this system's lists are still valid
@@ -609,204 +645,157 @@ __global__ void __launch_bounds__(32 * GROUP_ROW_WARPS)
   const int counts[3] = {s.cell_counts[0], s.cell_counts[1], s.cell_counts[2]};
   const int cells = counts[0] * counts[1] * counts[2];
   const int *gstart = cell_gstart + s.cell_start_base;
+  const int *cstart = cell_start + s.cell_start_base;
+  const int first_lane = part == 0 && lane == 0;
   if (q >= gstart[cells]) {  // an unused slot (the cells hold fewer groups than allocated)
-    if (threadIdx.x == 0) {
+    if (first_lane) {
       gsize[warp] = 0;
       gnbr_count[warp] = 0;
     }
     return;
   }
-  if (threadIdx.x == 0) row_count = 0;
-  __syncthreads();
-  int lo = 0, hi = cells;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (gstart[mid] <= q) lo = mid; else hi = mid;
+  const int cell0 = group_cell[warp];
+  const int o0 = s.atom_start + cstart[cell0] + (q - gstart[cell0]) * G;
+  const int size = min(G, s.atom_start + cstart[cell0 + 1] - o0);
+  const float4 origin0 = spos[o0];
+  const float4 box_lo = group_box[2 * warp], box_hi = group_box[2 * warp + 1];  // wrapped coordinates
+  if (part == 0 && lane < G) {
+    // the group's atoms measured from its first (an absent one, a copy of it): -2 x_a and |x_a|^2;
+    // their indices and the range of their excluded partners
+    const bool valid = lane < size;
+    const int si = o0 + (valid ? lane : 0), i = slot_info[si].y;
+    const float4 pw = spos[si];
+    if (valid) origin[i] = posq[i];  // skin check origin
+    const int e_lo = valid ? excl_start[i] : 0, e_hi = valid ? excl_start[i + 1] : 0;
+    const float dx = pw.x - origin0.x, dy = pw.y - origin0.y, dz = pw.z - origin0.z;
+    group_near[rib][lane] = make_float4(-2.f * dx, -2.f * dy, -2.f * dz, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+    excluded[rib][lane] = make_int4(i, e_lo < e_hi ? excl_partners[e_lo] : INT_MAX,
+                                    e_lo < e_hi ? excl_partners[e_hi - 1] : INT_MIN, 0);
+    if (lane == 0) row_count[rib] = 0;
   }
-  const int cell0 = lo;
-  const int cbegin = s.atom_start + cell_start[s.cell_start_base + cell0];
-  const int cend = s.atom_start + cell_start[s.cell_start_base + cell0 + 1];
-  const int o0 = cbegin + (q - gstart[cell0]) * G;
-  const int size = min(G, cend - o0);
-  // every lane holds atom lane % G of the group
-  const int a = lane % G;
-  const bool valid = a < size;
-  const int si = valid ? group_order[o0 + a] : group_order[o0];
-  const int i = slot_info[si].y;
-  const float4 pw = spos[si];
-  if (valid && threadIdx.x < G) origin[i] = posq[i];  // skin check origin
-  const int e_lo = valid ? excl_start[i] : 0, e_hi = valid ? excl_start[i + 1] : 0;
-  const int p_min = e_lo < e_hi ? excl_partners[e_lo] : INT_MAX;
-  const int p_max = e_lo < e_hi ? excl_partners[e_hi - 1] : INT_MIN;
-  int atom_i[G], atom_lo[G], atom_hi[G];
-#pragma unroll
-  for (int b = 0; b < G; ++b) {
-    atom_i[b] = __shfl_sync(0xffffffffu, i, b);
-    atom_lo[b] = __shfl_sync(0xffffffffu, p_min, b);
-    atom_hi[b] = __shfl_sync(0xffffffffu, p_max, b);
-  }
+  if (WARPS > 1) __syncthreads();
+  else __syncwarp();
   const unsigned absent = 0xFu & ~((1u << size) - 1u);  // atoms past the end of a short group
-  // the group's bounding box (wrapped coordinates)
-  float blo[3], bhi[3];
-  {
-    const float c[3] = {pw.x, pw.y, pw.z};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      float lo_d = valid ? c[d] : INFINITY, hi_d = valid ? c[d] : -INFINITY;
-#pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) {
-        lo_d = fminf(lo_d, __shfl_xor_sync(0xffffffffu, lo_d, o));
-        hi_d = fmaxf(hi_d, __shfl_xor_sync(0xffffffffu, hi_d, o));
-      }
-      blo[d] = lo_d;
-      bhi[d] = hi_d;
-    }
-  }
   const int cc[3] = {cell0 / (counts[1] * counts[2]), (cell0 / counts[2]) % counts[1], cell0 % counts[2]};
-  int base[3], count[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    base[d] = counts[d] >= 3 ? -1 : 0;
-    count[d] = counts[d] >= 3 ? 3 : (counts[d] == 2 ? 2 : 1);
-  }
-  const bool stencil_shift = counts[0] >= 3 && counts[1] >= 3 && counts[2] >= 3;
   const bool rectangular = s.box[3] == 0.f && s.box[6] == 0.f && s.box[7] == 0.f;
-  const float wcell[3] = {s.box[0] / counts[0], s.box[4] / counts[1], s.box[8] / counts[2]};
   const float cull2 = s.list_cutoff2 * 1.00004f * 1.0001f;  // the margin k_neighbours culls with
   const int cap = s.nbr_capacity;
   int *row = gnbr + s.gnbr_base + (long long)q * cap;
-  const int stencil_cells = count[0] * count[1] * count[2];
-  // the stencil's cells that need a search are dealt to the warps in turn (a cell before the
-  // group's own holds only atoms earlier in search order, whose groups list those pairs; in the
-  // shifted stencil of a rectangular box a cell beyond the list cutoff of the group's box is
-  // skipped), so the warps of a block get even shares: lane sc decides for stencil cell sc
-  // (at most 27), and the needed cells' ranks deal them out
-  bool need = false;
-  if (lane < stencil_cells) {
-    const int ox = lane / (count[1] * count[2]), oy = (lane / count[2]) % count[1], oz = lane % count[2];
-    const int rx = cc[0] + base[0] + ox, ry = cc[1] + base[1] + oy, rz = cc[2] + base[2] + oz;
-    const int cx = rx - (rx < 0 ? -1 : (rx >= counts[0] ? 1 : 0)) * counts[0];
-    const int cy = ry - (ry < 0 ? -1 : (ry >= counts[1] ? 1 : 0)) * counts[1];
-    const int cz = rz - (rz < 0 ? -1 : (rz >= counts[2] ? 1 : 0)) * counts[2];
-    need = (cx * counts[1] + cy) * counts[2] + cz >= cell0;
-    if (need && stencil_shift && rectangular) {
-      const float r[3] = {(float)rx, (float)ry, (float)rz};
+  // visits an axis: its three stencil cells (each through its own wrap), or every cell of an axis of
+  // fewer through each of three images
+  const int v0 = counts[0] >= 3 ? 3 : 3 * counts[0], v1 = counts[1] >= 3 ? 3 : 3 * counts[1],
+            v2 = counts[2] >= 3 ? 3 : 3 * counts[2];
+  int dealt = 0, found = 0;
+  for (int v = 0; v < v0 * v1 * v2; v += 32) {
+    bool need = v + lane < v0 * v1 * v2;
+    int code = 0, vg0 = 0, vg1 = 0, vbegin = 0, vend = 0;
+    if (need) {
+      const int t = v + lane, t2 = t / v2;
+      const int along[3] = {t2 / v1, t2 % v1, t % v2};
+      int c[3], image[3];
       float d2 = 0.f;
+      const float lo[3] = {box_lo.x, box_lo.y, box_lo.z}, hi[3] = {box_hi.x, box_hi.y, box_hi.z};
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const float clo = r[d] * wcell[d], chi = clo + wcell[d];
-        const float e = fmaxf(fmaxf(clo - bhi[d], blo[d] - chi), 0.f);
+        const int n = counts[d];
+        const int r = n >= 3 ? cc[d] - 1 + along[d] : along[d] - n;  // the cell's place, images included
+        image[d] = r < 0 ? -1 : (r >= n ? 1 : 0);
+        c[d] = r - image[d] * n;
+        const float width = s.box[4 * d] / n, clo = r * width;
+        const float e = fmaxf(fmaxf(clo - hi[d], lo[d] - (clo + width)), 0.f);
         d2 = fmaf(e, e, d2);
       }
-      need = d2 <= cull2;
+      const int cell = (c[0] * counts[1] + c[1]) * counts[2] + c[2];
+      need = cell >= cell0 && (!rectangular || d2 <= cull2);
+      if (need) {
+        code = shift_code(image[0], image[1], image[2]);
+        vg0 = s.group_base + gstart[cell];
+        vg1 = s.group_base + gstart[cell + 1];
+        vbegin = s.atom_start + cstart[cell];
+        vend = s.atom_start + cstart[cell + 1];
+      }
     }
-  }
-  const unsigned need_mask = __ballot_sync(0xffffffffu, need);
-  const int rank = __popc(need_mask & ((1u << lane) - 1u));
-  for (unsigned mine = __ballot_sync(0xffffffffu, need && rank % GROUP_ROW_WARPS == wib); mine; mine &= mine - 1u) {
-    const int sc = __ffs(mine) - 1;
-    const int ox = sc / (count[1] * count[2]), oy = (sc / count[2]) % count[1], oz = sc % count[2];
-    {
-      const int rx = cc[0] + base[0] + ox;
-      const int wx = rx < 0 ? -1 : (rx >= counts[0] ? 1 : 0);
-      const int cx = rx - wx * counts[0];
-      const int ry = cc[1] + base[1] + oy;
-      const int wy = ry < 0 ? -1 : (ry >= counts[1] ? 1 : 0);
-      const int cy = ry - wy * counts[1];
-      {
-        const int rz = cc[2] + base[2] + oz;
-        const int wz = rz < 0 ? -1 : (rz >= counts[2] ? 1 : 0);
-        const int cz = rz - wz * counts[2];
-        const int cell = (cx * counts[1] + cy) * counts[2] + cz;
-        const int begin = s.atom_start + cell_start[s.cell_start_base + cell];
-        const int end = s.atom_start + cell_start[s.cell_start_base + cell + 1];
-        // the lattice images to search this cell through: the stencil's own wrap on an axis
-        // with three cells or more, each of -1, 0, +1 on the others
-        const int na = counts[0] >= 3 ? 1 : 3, nb = counts[1] >= 3 ? 1 : 3, nc = counts[2] >= 3 ? 1 : 3;
-        for (int image = 0; image < na * nb * nc; ++image) {
-          const int ka = counts[0] >= 3 ? wx : image / (nb * nc) - 1;
-          const int kb = counts[1] >= 3 ? wy : (image / nc) % nb - 1;
-          const int kc = counts[2] >= 3 ? wz : image % nc - 1;
-          const int code = shift_code(ka, kb, kc);
-          const float4 S = s.shift[code];
-          const float slo[3] = {blo[0] - S.x, blo[1] - S.y, blo[2] - S.z};
-          const float shi[3] = {bhi[0] - S.x, bhi[1] - S.y, bhi[2] - S.z};
-          // the cell's groups, 32 at a time: a group before this one (its pairs with this group
-          // are in its own row) or whose box is beyond the list cutoff of this group's box is
-          // dropped whole; the atoms of the others are tested one by one, 8 groups at a time
-          const int gs0 = s.group_base + gstart[cell], gs1 = s.group_base + gstart[cell + 1];
-          for (int gb = max(gs0, warp); gb < gs1; gb += 32) {
-            const int gq = gb + lane;
-            bool near = gq < gs1;
-            if (near) {
-              const float4 lo2 = group_box[2 * gq], hi2 = group_box[2 * gq + 1];
-              const float l2[3] = {lo2.x, lo2.y, lo2.z}, h2[3] = {hi2.x, hi2.y, hi2.z};
-              float d2 = 0.f;
+    const unsigned need_mask = __ballot_sync(0xffffffffu, need);
+    const int rank = dealt + __popc(need_mask & ((1u << lane) - 1u));
+    dealt += __popc(need_mask);
+    unsigned mine = WARPS == 1 ? need_mask : __ballot_sync(0xffffffffu, need && rank % WARPS == part);
+    for (; mine; mine &= mine - 1u) {
+      const int from = __ffs(mine) - 1;
+      const int icode = __shfl_sync(0xffffffffu, code, from);
+      const int gs0 = __shfl_sync(0xffffffffu, vg0, from), gs1 = __shfl_sync(0xffffffffu, vg1, from);
+      const int begin = __shfl_sync(0xffffffffu, vbegin, from), end = __shfl_sync(0xffffffffu, vend, from);
+      const float4 S = s.shift[icode];
+      // the cell's groups, 32 at a time: a group before this one (its pairs with this group
+      // are in its own row) or whose box is beyond the list cutoff of this group's box is
+      // dropped whole; the atoms of the others are tested one by one, 8 groups at a time
+      for (int gb = max(gs0, warp); gb < gs1; gb += 32) {
+        const int gq = gb + lane;
+        bool near = gq < gs1;
+        if (near) {
+          const float4 lo2 = group_box[2 * gq], hi2 = group_box[2 * gq + 1];
+          const float ex = fmaxf(fmaxf(box_lo.x - S.x - hi2.x, lo2.x - (box_hi.x - S.x)), 0.f);
+          const float ey = fmaxf(fmaxf(box_lo.y - S.y - hi2.y, lo2.y - (box_hi.y - S.y)), 0.f);
+          const float ez = fmaxf(fmaxf(box_lo.z - S.z - hi2.z, lo2.z - (box_hi.z - S.z)), 0.f);
+          near = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= cull2;
+        }
+        const unsigned near_mask = __ballot_sync(0xffffffffu, near);
+        if (near) survivors[wib][__popc(near_mask & ((1u << lane) - 1u))] = begin + (gq - gs0) * G;
+        __syncwarp();
+        const int n_near = __popc(near_mask);
+        for (int t0 = 0; t0 < n_near; t0 += 8) {
+          const int t = t0 + (lane >> 2);
+          unsigned mask = 0;
+          const int g = (t < n_near ? survivors[wib][t] : end) + (lane & 3);
+          bool keep = g < end;
+          if (keep) {
+            // within the list cutoff of one of the group's atoms: with p and the atoms x_a
+            // measured from x_0, |p - x_a|^2 = |p|^2 + (|x_a|^2 - 2 x_a.p), least over a
+            const float4 pj = spos[g];
+            const float px = pj.x + S.x - origin0.x, py = pj.y + S.y - origin0.y, pz = pj.z + S.z - origin0.z;
+            float least = 0.f;
 #pragma unroll
-              for (int d = 0; d < 3; ++d) {
-                const float e = fmaxf(fmaxf(slo[d] - h2[d], l2[d] - shi[d]), 0.f);
-                d2 = fmaf(e, e, d2);
-              }
-              near = d2 <= cull2;
+            for (int u = 1; u < G; ++u) {
+              const float4 x = group_near[rib][u];
+              least = fminf(least, fmaf(px, x.x, fmaf(py, x.y, fmaf(pz, x.z, x.w))));
             }
-            const unsigned near_mask = __ballot_sync(0xffffffffu, near);
-            if (near) survivors[wib][__popc(near_mask & ((1u << lane) - 1u))] = gq;
-            __syncwarp();
-            const int n_near = __popc(near_mask);
-            for (int t0 = 0; t0 < n_near; t0 += 8) {
-              const int t = t0 + (lane >> 2);
-              bool keep = t < n_near;
-              unsigned mask = 0;
-              int g = 0;
-              if (keep) {
-                const int opos = begin + (survivors[wib][t] - gs0) * G + (lane & 3);
-                keep = opos < end;
-                if (keep) {
-                  g = group_order[opos];
-                  const float4 pj = spos[g];
-                  const float c[3] = {pj.x, pj.y, pj.z};
-                  float d2 = 0.f;
+            keep = fmaf(px, px, fmaf(py, py, fmaf(pz, pz, least))) <= cull2;
+          }
+          if (keep) {
+            // a later group's atom, or one of this group's own: earlier atoms only
+            if (g < o0 + G) mask = 0xFu & ~((1u << (g - o0)) - 1u);
+            const int j = slot_info[g].y;
 #pragma unroll
-                  for (int d = 0; d < 3; ++d) {
-                    const float e = fmaxf(fmaxf(slo[d] - c[d], c[d] - shi[d]), 0.f);
-                    d2 = fmaf(e, e, d2);
-                  }
-                  keep = d2 <= cull2;
-                }
-                if (keep) {
-                  // a later group's atom, or one of this group's own: earlier atoms only
-                  if (opos < o0 + G) mask = 0xFu & ~((1u << (opos - o0)) - 1u);
-                  const int j = slot_info[g].y;
-#pragma unroll
-                  for (int u = 0; u < G; ++u)
-                    if (j >= atom_lo[u] && j <= atom_hi[u] && is_excluded(excl_start, excl_partners, atom_i[u], j))
-                      mask |= 1u << u;
-                  mask |= absent;
-                  keep = mask != 0xFu;
-                }
-              }
-              const unsigned hits = __ballot_sync(0xffffffffu, keep);
-              if (hits) {
-                int at = 0;
-                if (lane == 0) at = atomicAdd(&row_count, __popc(hits));
-                at = __shfl_sync(0xffffffffu, at, 0) + __popc(hits & ((1u << lane) - 1u));
-                if (keep && at < cap)
-                  row[at] = (int)((unsigned)g | ((unsigned)code << GROUP_CODE_SHIFT) | (mask << GROUP_MASK_SHIFT));
-              }
+            for (int u = 0; u < G; ++u) {
+              const int4 x = excluded[rib][u];
+              if (j >= x.y && j <= x.z && is_excluded(excl_start, excl_partners, x.x, j)) mask |= 1u << u;
             }
-            __syncwarp();
+            mask |= absent;
+            keep = mask != 0xFu;
+          }
+          const unsigned hits = __ballot_sync(0xffffffffu, keep);
+          if (hits) {
+            int at = found;
+            if (WARPS > 1) {
+              if (lane == 0) at = atomicAdd(&row_count[rib], __popc(hits));
+              at = __shfl_sync(0xffffffffu, at, 0);
+            }
+            found += __popc(hits);
+            at += __popc(hits & ((1u << lane) - 1u));
+            if (keep && at < cap)
+              row[at] = (int)((unsigned)g | ((unsigned)icode << GROUP_CODE_SHIFT) | (mask << GROUP_MASK_SHIFT));
           }
         }
+        __syncwarp();
       }
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int found = row_count;
-    gnbr_count[warp] = min(found, cap);
+  if (WARPS > 1) __syncthreads();
+  if (first_lane) {
+    const int total = WARPS > 1 ? row_count[rib] : found;
+    gnbr_count[warp] = min(total, cap);
     gfirst[warp] = o0;
     gsize[warp] = size;
-    atomicMax(&required[sidx], found);
+    atomicMax(&required[sidx], total);
   }
 }
 
@@ -902,21 +891,27 @@ void launch_rebuild(const LaunchCtx &ctx, cudaStream_t stream) {
                                                          ctx.cell_start, ctx.cell_count,
                                                          ctx.cell_atoms, n, only);
   LaunchCtxView v{ctx.posq,      ctx.atom_type, ctx.spos,      ctx.wrap,      ctx.sorted_orig,
-                  ctx.sorted_type, ctx.rank,   ctx.group_order, ctx.slot_info, ctx.order_pos,
-                  ctx.pair_list != 1 ? ctx.group_box : nullptr, ctx.cell_gstart};
+                  ctx.sorted_type, ctx.rank,   ctx.group_order, ctx.slot_info,
+                  ctx.pair_list != 1 ? ctx.group_box : nullptr, ctx.cell_gstart, ctx.group_cell};
   k_cells_sort<<<ctx.n_cells_total, 256, 0, stream>>>(ctx.cell_sys, ctx.sys, ctx.cell_start,
                                                       ctx.cell_count, ctx.cell_atoms, v, only);
   const int blocks = (ctx.n_groups_total + NBR_WARPS - 1) / NBR_WARPS;
   if (ctx.pair_list != 1) {  // group-pair rows (the cell scan counted 4-atom groups)
-    k_group_rows<<<ctx.n_groups_total, 32 * GROUP_ROW_WARPS, 0, stream>>>(
-        ctx.posq, ctx.group_sys, ctx.sys, ctx.cell_start, ctx.cell_gstart, ctx.group_order, ctx.excl_start,
-        ctx.excl_partners, ctx.spos, ctx.slot_info, ctx.group_box, ctx.gnbr, ctx.gnbr_count, ctx.gfirst, ctx.gsize,
-        ctx.required + ctx.n_systems, ctx.origin, ctx.n_groups_total, only);
+    auto rows = [&](auto kernel, int blocks, int threads) {
+      kernel<<<blocks, threads, 0, stream>>>(
+          ctx.posq, ctx.group_sys, ctx.sys, ctx.cell_start, ctx.cell_gstart, ctx.group_cell, ctx.excl_start,
+          ctx.excl_partners, ctx.spos, ctx.slot_info, ctx.group_box, ctx.gnbr, ctx.gnbr_count, ctx.gfirst, ctx.gsize,
+          ctx.required + ctx.n_systems, ctx.origin, ctx.n_groups_total, only);
+    };
+    const int n_groups = ctx.n_groups_total;
+    if (n_groups >= GROUP_ROW_WARP_GROUPS) rows(k_group_rows<1>, (n_groups + 3) / 4, 128);
+    else if (n_groups >= GROUP_ROW_BLOCK_GROUPS) rows(k_group_rows<4>, n_groups, 128);
+    else rows(k_group_rows<8>, n_groups, 256);
     if (ctx.pair_list != 2) return;
   }
 #define RMD_NBR_ARGS                                                                                      \
   ctx.posq, ctx.group_sys, ctx.sys, ctx.cell_start, ctx.cell_gstart, ctx.group_order, ctx.excl_start,  \
-      ctx.excl_partners, ctx.spos, ctx.sorted_orig, ctx.nbr, ctx.nbr_count, ctx.required, ctx.origin, \
+      ctx.excl_partners, ctx.spos, ctx.sorted_orig, ctx.pair_list == 2 ? ctx.cell_atoms : nullptr, ctx.rank, ctx.nbr, ctx.nbr_count, ctx.required, ctx.origin, \
       ctx.n_groups_total, only
   // 4-atom groups too few to fill the GPU with one warp each (a box of a few thousand atoms)
   // search three warps a group; otherwise one warp a group keeps more groups resident

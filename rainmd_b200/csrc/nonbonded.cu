@@ -222,9 +222,8 @@ __global__ void __launch_bounds__(128) k_nonbonded(
 // ------------------------------------------------------------------ group-pair kernel
 // The same pair physics over the group-pair rows (lists.cu k_group_rows). A row's entries are
 // dealt to the lanes of `split` warps, one partner a lane. A lane first tests its partner's
-// squared distances to the group's GROUP_ATOMS atoms (their records are in the warp's shared
-// memory); the entries with an unmasked atom within the cutoff queue in a per-warp ring, and
-// each batch of 32 queued entries is evaluated one entry a lane, the partner against the four
+// least squared distance to the group's GROUP_ATOMS atoms, in an expanded form of three
+// multiply-adds an atom; the entries within the cutoff queue in a per-warp ring, and each batch of 32 queued entries is evaluated one entry a lane, the partner against the four
 // atoms in turn, so a batch evaluates 128 pairs of which none belongs to an entry beyond the
 // cutoff of all four (about half the rows' entries). Each pair is evaluated once, from the
 // group that lists it. Its force is quantised to 64-bit fixed point
@@ -328,7 +327,7 @@ __device__ __forceinline__ void group_pair_entry(const unsigned e, const float4 
 template <bool ENERGY>
 __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
     const float4 *__restrict__ posq, const float4 *__restrict__ spos, const int2 *__restrict__ slot_info,
-    const int *__restrict__ group_order, const int *__restrict__ group_sys, const DevSys *__restrict__ sys,
+    const int *__restrict__ group_sys, const DevSys *__restrict__ sys,
     const float2 *__restrict__ lj, const int *__restrict__ gnbr, const int *__restrict__ gnbr_count,
     const int *__restrict__ gfirst, const int *__restrict__ gsize, const int *__restrict__ exc_start,
     const int *__restrict__ exc_partner, const float4 *__restrict__ exc_param,
@@ -353,21 +352,32 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   // records in this warp's shared memory, their original indices in registers
   __shared__ float4 group_pos[4][G];
   __shared__ int group_lj[4][G];
+  __shared__ float4 group_near[4][G];
   const int wib = threadIdx.x >> 5;
   int ia[G];
+  const float4 p0 = spos[first];
+  // the entry test's coefficients: with a partner p and the group's atoms x_a measured from x_0,
+  // |p - x_a|^2 = |p|^2 + (|x_a|^2 - 2 x_a.p) (an absent atom is a copy of x_0)
 #pragma unroll
   for (int a = 0; a < G; ++a) {
-    const int si = group_order[first + (a < size ? a : 0)];
-    ia[a] = slot_info[si].y;
+    const int si = first + (a < size ? a : 0);
+    const int2 info = slot_info[si];
+    const float4 pa = spos[si];
+    ia[a] = info.y;
     if (lane == a) {
-      group_pos[wib][a] = spos[si];
-      group_lj[wib][a] = slot_info[si].x * s.type_count;
+      group_pos[wib][a] = pa;
+      group_lj[wib][a] = info.x * s.type_count;
+      const float dx = pa.x - p0.x, dy = pa.y - p0.y, dz = pa.z - p0.z;
+      group_near[wib][a] = make_float4(-2.f * dx, -2.f * dy, -2.f * dz, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
     }
   }
   __syncwarp();
   const float alpha = s.alpha;
   const float gauss_k = 2.0f * alpha * 0.5641895835477563f;  // 2a/sqrt(pi)
   const float cut2 = s.cutoff2;
+  // the test's own rounding (coordinates of up to the box's size) stays below this margin, and an
+  // entry it lets in needlessly contributes zero
+  const float near2 = cut2 * 1.0001f;
   const int *row = gnbr + s.gnbr_base + (long long)(warp - s.group_base) * s.nbr_capacity;
   // per group atom: force x, y, z (and energies lj, coulomb, virial) in fixed point
   long long acc[G][ENERGY ? 6 : 3];
@@ -377,8 +387,8 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
     for (int c = 0; c < (ENERGY ? 6 : 3); ++c) acc[a][c] = 0;
   const int stride = 32 * split;
   int k = 32 * part + lane;
-  // Each pass first tests its 32 entries with the four squared distances alone; an entry with
-  // some unmasked group atom within the cutoff joins this warp's ring in shared memory (about
+  // Each pass first tests its 32 entries' distances alone; an entry with some group atom within
+  // the cutoff joins this warp's ring in shared memory (about
   // half of them: the rows hold every partner within the list cutoff of the group's box), and
   // whenever 32 are queued the warp evaluates them, one entry a lane, so the full pair
   // arithmetic runs on entries that contribute. The queued entries keep their records, so
@@ -474,14 +484,14 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
       S1 = s.shift[(e1 >> GROUP_CODE_SHIFT) & 31u];
       e2 = k + 2 * stride < count ? (unsigned)__ldg(row + k + 2 * stride) : NO_ENTRY;
     }
-    bool any = false;
+    const float px = pj.x + S.x - p0.x, py = pj.y + S.y - p0.y, pz = pj.z + S.z - p0.z;
+    float least = 0.f;
 #pragma unroll
-    for (int a = 0; a < G; ++a) {
-      const float4 pw = group_pos[wib][a];
-      const float3 d = make_float3(pw.x - pj.x - S.x, pw.y - pj.y - S.y, pw.z - pj.z - S.z);
-      const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-      any |= !((e >> (GROUP_MASK_SHIFT + a)) & 1u) && r2 <= cut2;
+    for (int a = 1; a < G; ++a) {
+      const float4 near = group_near[wib][a];
+      least = fminf(least, fmaf(px, near.x, fmaf(py, near.y, fmaf(pz, near.z, near.w))));
     }
+    const bool any = k < count && fmaf(px, px, fmaf(py, py, fmaf(pz, pz, least))) <= near2;
     const unsigned hits = __ballot_sync(0xffffffffu, any);
     if (any) {
       const int slot = (head + queued + __popc(hits & ((1u << lane) - 1u))) & 63;
@@ -565,13 +575,13 @@ static void launch_group_pairs(const LaunchCtx &c, bool energy, int lanes, cudaS
   const size_t smem = sizeof(float2) * lj_entries;
   if (energy) {
     k_group_pairs<true><<<blocks, threads, smem, stream>>>(
-        c.posq, c.spos, c.slot_info, c.group_order, c.group_sys, c.sys, c.lj, c.gnbr, c.gnbr_count, c.gfirst,
+        c.posq, c.spos, c.slot_info, c.group_sys, c.sys, c.lj, c.gnbr, c.gnbr_count, c.gfirst,
         c.gsize, c.exc_start, c.exc_partner, c.exc_param, c.force, c.e_acc, c.n_atoms, c.n_groups_total, lj_entries,
         split);
     k_group_pair_energies<<<(c.n_atoms + 255) / 256, 256, 0, stream>>>(c.e_acc, c.e_lj, c.e_coul, c.e_vir, c.n_atoms);
   } else {
     k_group_pairs<false><<<blocks, threads, smem, stream>>>(
-        c.posq, c.spos, c.slot_info, c.group_order, c.group_sys, c.sys, c.lj, c.gnbr, c.gnbr_count, c.gfirst,
+        c.posq, c.spos, c.slot_info, c.group_sys, c.sys, c.lj, c.gnbr, c.gnbr_count, c.gfirst,
         c.gsize, c.exc_start, c.exc_partner, c.exc_param, c.force, c.e_acc, c.n_atoms, c.n_groups_total, lj_entries,
         split);
   }

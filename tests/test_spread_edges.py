@@ -19,18 +19,13 @@ def test_atoms_on_the_faces(order, grid):
     s, pos, _ = system_for("ala-wat")
     box = np.asarray(s["boxVectors"]).reshape(3, 3)
     pos = np.asarray(pos, dtype=np.float64).reshape(-1, 3).copy()
-    # whole molecules: shift each so that its first atom sits on a face, an edge or a corner, or
-    # three cells away
+    # everything moved so that an atom sits on a corner of the cell (or a rounding step before one), then
+    # whole molecules by whole cells, some far outside
     molecule = np.asarray(s["topology"]["moleculeOfAtom"])
-    first = {}
-    for k, m in enumerate(molecule):
-        first.setdefault(int(m), k)
-    targets = [np.array(t) @ box for t in ([0, 0, 0], [1, 0, 0], [1, 1, 1], [1 - 2.0 ** -24, 0, 1], [-3, 2, 0], [4, -2, 3])]
-    shifts = {m: np.round((targets[m % 6] - pos[k]) @ np.linalg.inv(box)) @ box for m, k in first.items()}
-    pos += np.array([shifts[int(m)] for m in molecule])
-    for m in range(1, 6):  # five waters moved whole onto the targets themselves (their pairs change too)
-        rows = molecule == m + 20
-        pos[rows] += targets[m] - pos[np.nonzero(rows)[0][0]]
+    corner = np.array([1.0, 1 - 2.0 ** -24, 0.0]) @ box
+    pos += corner - pos[30]
+    cells = np.array([[0, 0, 0], [-3, 2, 0], [4, -2, 3], [0, 0, -1]])
+    pos += (cells[molecule % 4] @ box)
     flat = pos.reshape(-1)
     sim = engine_for(s, flat, grid=list(grid), pmeOrder=order, neighbourSlack=4.0)
     e, _ = sim.debugEvaluate()
