@@ -17,6 +17,7 @@
 // list pairs (the barostat surrogate's input), are only computed in the ENERGY variant.
 #include "common.cuh"
 #include "kernels.h"
+#include "pair.cuh"
 
 namespace rmd {
 
@@ -100,19 +101,11 @@ __global__ void __launch_bounds__(128) k_nonbonded(
       if (k + 2 * LANES < count) e2 = (unsigned)__ldg(row + k + 2 * LANES);
     }
     const float3 d = make_float3(pw.x - pj.x - S.x, pw.y - pj.y - S.y, pw.z - pj.z - S.z);
-    const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
+    const float r2 = pair_r2(d.x, d.y, d.z);
     if (r2 <= cut2) {
-      const float inv_r = rsqrt_refined(r2);
-      const float inv_r2 = inv_r * inv_r;
-      const float inv_r6 = inv_r2 * inv_r2 * inv_r2;
       const float2 ab = ljrow[tj];
-      const float a12 = ab.x * inv_r6 * inv_r6, b6 = ab.y * inv_r6;
-      float scalar = (12.0f * a12 - 6.0f * b6) * inv_r2;
-      const float qq = (float)ONE_4PI_EPS0 * (pw.w * pj.w);  // symmetric in i and j
-      const float r = r2 * inv_r;
-      float gauss;
-      const float screened = erfc_and_gauss(alpha * r, gauss);
-      scalar = fmaf(qq * fmaf(screened, inv_r, gauss_k * gauss), inv_r2, scalar);
+      const PairTerms<float> t = pair_terms(r2, ab.x, ab.y, op_mul(pw.w, pj.w), alpha, gauss_k);  // symmetric in i and j
+      const float scalar = t.scalar;
       if (PAIR_FIXED) {
         qx += (long long)to_fixed(scalar * d.x);
         qy += (long long)to_fixed(scalar * d.y);
@@ -124,12 +117,12 @@ __global__ void __launch_bounds__(128) k_nonbonded(
       }
       if (ENERGY) {
         if (PAIR_FIXED) {
-          qlj += (long long)to_fixed(a12 - b6);
-          qcoul += (long long)to_fixed(qq * screened * inv_r);
+          qlj += (long long)to_fixed(op_add(t.a12, -t.b6));
+          qcoul += (long long)to_fixed(op_mul(t.charge, t.inv_r));
           qvir += (long long)to_fixed(scalar * r2);
         } else {
-          elj += a12 - b6;
-          ecoul = fmaf(qq * screened, inv_r, ecoul);
+          elj += t.a12 - t.b6;
+          ecoul = fmaf(t.charge, t.inv_r, ecoul);
           evir = fmaf(scalar, r2, evir);
         }
       }
@@ -258,59 +251,70 @@ __device__ __forceinline__ long long warp_sum_sixteen(long long (&v)[16], int la
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// One row entry against the group's GROUP_ATOMS atoms: the four pairs are evaluated without
-// branches (a pair that is masked or beyond the cutoff is evaluated at r = 1 nm and contributes
-// zero), so their chains can interleave. Each pair force is quantised (the scale folded into
-// the scalar factor: a power of two, so the product rounds exactly as the scaled force does)
-// and added to the group atom's integer sums in `acc`; the partner gets the negated sum with
-// one 64-bit atomic per component (energies as they are).
+// One row entry against the group's GROUP_ATOMS atoms, two at a time (pair.cuh Pair2). The pairs are
+// evaluated without branches, so their chains can interleave; a pair that is masked or beyond the
+// cutoff contributes zero (whatever its own arithmetic gave, an excluded pair's r = 0 included).
+// Each pair force is quantised (the scale folded into the scalar factor: a power of two, so the
+// product rounds exactly as the scaled force does) and added to the group atom's integer sums in
+// `acc`; the partner gets the negated sum with one 64-bit atomic per component (energies as they
+// are). gpos: the four atoms' x, y, z and charge, component by component.
 template <bool ENERGY>
 __device__ __forceinline__ void group_pair_entry(const unsigned e, const float4 pj, const int2 info_j,
-                                                 const float4 *__restrict__ gpos, const int *__restrict__ glj,
+                                                 const float *__restrict__ gpos, const int *__restrict__ glj,
                                                  const float2 *__restrict__ ljtab, const DevSys &s, float alpha,
                                                  float gauss_k, float cut2, long long (&acc)[GROUP_ATOMS][ENERGY ? 6 : 3],
                                                  unsigned long long *__restrict__ force,
                                                  unsigned long long *__restrict__ e_acc, int n_atoms) {
   const float4 S = s.shift[(e >> GROUP_CODE_SHIFT) & 31u];
+  const Pair2 jnx = pack2(-pj.x, -pj.x), jny = pack2(-pj.y, -pj.y), jnz = pack2(-pj.z, -pj.z), qj = pack2(pj.w, pj.w);
+  const Pair2 Snx = pack2(-S.x, -S.x), Sny = pack2(-S.y, -S.y), Snz = pack2(-S.z, -S.z);
+  const Pair2 alpha2 = pack2(alpha, alpha), gauss2 = pack2(gauss_k, gauss_k);
   long long jx = 0, jy = 0, jz = 0, jl = 0, jc = 0, jv = 0;
 #pragma unroll
-  for (int a = 0; a < GROUP_ATOMS; ++a) {
-    const float4 pw = gpos[a];
-    const float3 d = make_float3(pw.x - pj.x - S.x, pw.y - pj.y - S.y, pw.z - pj.z - S.z);
-    const float r2d = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-    const bool in = !((e >> (GROUP_MASK_SHIFT + a)) & 1u) && r2d <= cut2;
-    const float r2 = in ? r2d : 1.0f;
-    const float inv_r = rsqrt_refined(r2);
-    const float inv_r2 = inv_r * inv_r;
-    const float inv_r6 = inv_r2 * inv_r2 * inv_r2;
-    const float2 ab = ljtab[glj[a] + info_j.x];
-    const float a12 = ab.x * inv_r6 * inv_r6, b6 = ab.y * inv_r6;
-    float scalar = (12.0f * a12 - 6.0f * b6) * inv_r2;
-    const float qq = (float)ONE_4PI_EPS0 * (pw.w * pj.w);
-    const float r = r2 * inv_r;
-    float gauss;
-    const float screened = erfc_and_gauss(alpha * r, gauss);
-    scalar = fmaf(qq * fmaf(screened, inv_r, gauss_k * gauss), inv_r2, scalar);
-    scalar = in ? scalar * FORCE_SCALE_F : 0.0f;
-    const long long fx = __float2ll_rn(scalar * d.x);
-    const long long fy = __float2ll_rn(scalar * d.y);
-    const long long fz = __float2ll_rn(scalar * d.z);
-    acc[a][0] += fx;
-    acc[a][1] += fy;
-    acc[a][2] += fz;
-    jx += fx;
-    jy += fy;
-    jz += fz;
+  for (int h = 0; h < GROUP_ATOMS; h += 2) {
+    auto two = [&](int c) {
+      const float2 v = *reinterpret_cast<const float2 *>(gpos + GROUP_ATOMS * c + h);
+      return pack2(v.x, v.y);
+    };
+    const Pair2 dx = op_add(op_add(two(0), jnx), Snx), dy = op_add(op_add(two(1), jny), Sny),
+                dz = op_add(op_add(two(2), jnz), Snz);
+    const Pair2 r2 = pair_r2(dx, dy, dz);
+    const float2 ab0 = ljtab[glj[h] + info_j.x], ab1 = ljtab[glj[h + 1] + info_j.x];
+    const PairTerms<Pair2> t =
+        pair_terms(r2, pack2(ab0.x, ab1.x), pack2(ab0.y, ab1.y), op_mul(two(3), qj), alpha2, gauss2);
+    const float2 r2s = unpack2(r2), sc = unpack2(op_mul(t.scalar, op_const<Pair2>(FORCE_SCALE_F)));
+    const bool in[2] = {!((e >> (GROUP_MASK_SHIFT + h)) & 1u) && r2s.x <= cut2,
+                        !((e >> (GROUP_MASK_SHIFT + h + 1)) & 1u) && r2s.y <= cut2};
+    const float scalar[2] = {in[0] ? sc.x : 0.0f, in[1] ? sc.y : 0.0f};
+    const Pair2 scalar2 = pack2(scalar[0], scalar[1]);
+    const float2 fx = unpack2(op_mul(scalar2, dx)), fy = unpack2(op_mul(scalar2, dy)), fz = unpack2(op_mul(scalar2, dz));
+    float2 lj, coul;
     if (ENERGY) {
-      const long long el = in ? (long long)to_fixed(a12 - b6) : 0;
-      const long long ec = in ? (long long)to_fixed(qq * screened * inv_r) : 0;
-      const long long ev = __float2ll_rn(scalar * r2);
-      acc[a][ENERGY ? 3 : 0] += el;
-      acc[a][ENERGY ? 4 : 0] += ec;
-      acc[a][ENERGY ? 5 : 0] += ev;
-      jl += el;
-      jc += ec;
-      jv += ev;
+      lj = unpack2(op_fma(t.b6, op_const<Pair2>(-1.0f), t.a12));
+      coul = unpack2(op_mul(t.charge, t.inv_r));
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int a = h + k;
+      const long long qx = __float2ll_rn(k ? fx.y : fx.x), qy = __float2ll_rn(k ? fy.y : fy.x),
+                      qz = __float2ll_rn(k ? fz.y : fz.x);
+      acc[a][0] += qx;
+      acc[a][1] += qy;
+      acc[a][2] += qz;
+      jx += qx;
+      jy += qy;
+      jz += qz;
+      if (ENERGY) {
+        const long long el = in[k] ? (long long)to_fixed(k ? lj.y : lj.x) : 0;
+        const long long ec = in[k] ? (long long)to_fixed(k ? coul.y : coul.x) : 0;
+        const long long ev = in[k] ? __float2ll_rn(scalar[k] * (k ? r2s.y : r2s.x)) : 0;
+        acc[a][ENERGY ? 3 : 0] += el;
+        acc[a][ENERGY ? 4 : 0] += ec;
+        acc[a][ENERGY ? 5 : 0] += ev;
+        jl += el;
+        jc += ec;
+        jv += ev;
+      }
     }
   }
   const int j = info_j.y;
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   const float2 *ljtab = (lj_in_smem ? lj_shared : lj) + s.lj_base;
   // the group's atoms, the same for every lane (an absent atom is masked by every entry): their
   // records in this warp's shared memory, their original indices in registers
-  __shared__ float4 group_pos[4][G];
+  __shared__ __align__(16) float group_pos[4][4 * G];  // x, y, z, charge of each atom, component by component
   __shared__ int group_lj[4][G];
   __shared__ float4 group_near[4][G];
   const int wib = threadIdx.x >> 5;
@@ -365,7 +369,10 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
     const float4 pa = spos[si];
     ia[a] = info.y;
     if (lane == a) {
-      group_pos[wib][a] = pa;
+      group_pos[wib][a] = pa.x;
+      group_pos[wib][G + a] = pa.y;
+      group_pos[wib][2 * G + a] = pa.z;
+      group_pos[wib][3 * G + a] = pa.w;
       group_lj[wib][a] = info.x * s.type_count;
       const float dx = pa.x - p0.x, dy = pa.y - p0.y, dz = pa.z - p0.z;
       group_near[wib][a] = make_float4(-2.f * dx, -2.f * dy, -2.f * dz, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
