@@ -261,11 +261,12 @@ __device__ __forceinline__ long long warp_sum_sixteen(long long (&v)[16], int la
 template <bool ENERGY>
 __device__ __forceinline__ void group_pair_entry(const unsigned e, const float4 pj, const int2 info_j,
                                                  const float *__restrict__ gpos, const int *__restrict__ glj,
-                                                 const float2 *__restrict__ ljtab, const DevSys &s, float alpha,
-                                                 float gauss_k, float cut2, long long (&acc)[GROUP_ATOMS][ENERGY ? 6 : 3],
+                                                 const float2 *__restrict__ ljtab, const float4 *__restrict__ shift,
+                                                 float alpha, float gauss_k, float cut2,
+                                                 long long (&acc)[GROUP_ATOMS][ENERGY ? 6 : 3],
                                                  unsigned long long *__restrict__ force,
                                                  unsigned long long *__restrict__ e_acc, int n_atoms) {
-  const float4 S = s.shift[(e >> GROUP_CODE_SHIFT) & 31u];
+  const float4 S = shift[(e >> GROUP_CODE_SHIFT) & 31u];
   const Pair2 jnx = pack2(-pj.x, -pj.x), jny = pack2(-pj.y, -pj.y), jnz = pack2(-pj.z, -pj.z), qj = pack2(pj.w, pj.w);
   const Pair2 Snx = pack2(-S.x, -S.x), Sny = pack2(-S.y, -S.y), Snz = pack2(-S.z, -S.z);
   const Pair2 alpha2 = pack2(alpha, alpha), gauss2 = pack2(gauss_k, gauss_k);
@@ -328,6 +329,8 @@ __device__ __forceinline__ void group_pair_entry(const unsigned e, const float4 
   }
 }
 
+constexpr int PREFETCH_GROUPS = 48 * 1024;  // groups whose rows together pass about 80 MB
+
 template <bool ENERGY>
 __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
     const float4 *__restrict__ posq, const float4 *__restrict__ spos, const int2 *__restrict__ slot_info,
@@ -357,7 +360,18 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   __shared__ __align__(16) float group_pos[4][4 * G];  // x, y, z, charge of each atom, component by component
   __shared__ int group_lj[4][G];
   __shared__ float4 group_near[4][G];
+  // the system's lattice shifts, read twice an entry: from shared memory, since 32 lanes' reads of up
+  // to 27 records took the L1 as many wavefronts (250,000 atoms 429 -> 354 us, 99,999 160 -> 143, 23,558
+  // 46.7 -> 43.2, a batch of 24 124 -> 113)
+  __shared__ float4 shift[4][32];
   const int wib = threadIdx.x >> 5;
+  const int *row = gnbr + s.gnbr_base + (long long)(warp - s.group_base) * s.nbr_capacity;
+  // Rows too many for L2 are read from device memory: this one starts on its way while the records
+  // below are read (250,000 atoms 354 -> 341 us; 99,999 143.0 -> 143.9 and a batch 112.6 -> 114, whose
+  // rows stay in L2, hence the line).
+  if (n_groups >= PREFETCH_GROUPS)
+    for (int k = 32 * lane; k < count; k += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + k));
+  if (lane < 27) shift[wib][lane] = s.shift[lane];
   int ia[G];
   const float4 p0 = spos[first];
   // the entry test's coefficients: with a partner p and the group's atoms x_a measured from x_0,
@@ -385,7 +399,6 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   // the test's own rounding (coordinates of up to the box's size) stays below this margin, and an
   // entry it lets in needlessly contributes zero
   const float near2 = cut2 * 1.0001f;
-  const int *row = gnbr + s.gnbr_base + (long long)(warp - s.group_base) * s.nbr_capacity;
   // per group atom: force x, y, z (and energies lj, coulomb, virial) in fixed point
   long long acc[G][ENERGY ? 6 : 3];
 #pragma unroll
@@ -412,7 +425,6 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   unsigned e2 = k + stride < count ? (unsigned)__ldg(row + k + stride) : NO_ENTRY;
   float4 pj1 = __ldg(spos + (e1 & GROUP_SLOT_MASK));
   int2 info1 = __ldg(slot_info + (e1 & GROUP_SLOT_MASK));
-  float4 S1 = s.shift[(e1 >> GROUP_CODE_SHIFT) & 31u];
   // Exceptions of the group atoms (first warp of the row: lanes 8a .. 8a + 7 for atom a): 1-4
   // scaled LJ/Coulomb and -q_i q_j erf(a r)/r, no cutoff, exactly as the atom-row kernel
   // evaluates them. They come before the row walk, so their chain of dependent loads overlaps
@@ -482,13 +494,12 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   }
   for (int k0 = 32 * part; k0 < count; k0 += stride, k += stride) {
     const unsigned e = e1;
-    const float4 pj = pj1, S = S1;
+    const float4 pj = pj1, S = shift[wib][(e >> GROUP_CODE_SHIFT) & 31u];
     const int2 info_j = info1;
     if (k0 + stride < count) {
       e1 = e2;
       pj1 = __ldg(spos + (e1 & GROUP_SLOT_MASK));
       info1 = __ldg(slot_info + (e1 & GROUP_SLOT_MASK));
-      S1 = s.shift[(e1 >> GROUP_CODE_SHIFT) & 31u];
       e2 = k + 2 * stride < count ? (unsigned)__ldg(row + k + 2 * stride) : NO_ENTRY;
     }
     const float px = pj.x + S.x - p0.x, py = pj.y + S.y - p0.y, pz = pj.z + S.z - p0.z;
@@ -511,7 +522,7 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
       __syncwarp();
       const int slot = (head + lane) & 63;
       group_pair_entry<ENERGY>(ring_e[wib][slot], ring_p[wib][slot], ring_i[wib][slot], group_pos[wib],
-                               group_lj[wib], ljtab, s, alpha, gauss_k, cut2, acc, force, e_acc, n_atoms);
+                               group_lj[wib], ljtab, shift[wib], alpha, gauss_k, cut2, acc, force, e_acc, n_atoms);
       __syncwarp();  // every lane has read its slot before the next pass refills the ring
       head = (head + 32) & 63;
       queued -= 32;
@@ -523,7 +534,7 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
     const bool mine = lane < queued;
     group_pair_entry<ENERGY>(mine ? ring_e[wib][slot] : NO_ENTRY,
                              mine ? ring_p[wib][slot] : make_float4(0.f, 0.f, 0.f, 0.f),
-                             mine ? ring_i[wib][slot] : make_int2(0, 0), group_pos[wib], group_lj[wib], ljtab, s,
+                             mine ? ring_i[wib][slot] : make_int2(0, 0), group_pos[wib], group_lj[wib], ljtab, shift[wib],
                              alpha, gauss_k, cut2, acc, force, e_acc, n_atoms);
   }
   // the group atoms' sums over the warp: value 4a + c (component c of atom a) ends in lanes
