@@ -43,8 +43,11 @@ struct DevSys {
   int cell_capacity;    // cells allocated for this system
   int group_base;       // first neighbour-search group slot of this system
   long long nbr_base;   // offset of row 0 in the neighbour array
-  int nbr_capacity;     // entries a row holds (per-atom rows and group rows alike)
+  int nbr_capacity;     // entries a per-atom row holds; more than this in any row makes the host grow the lists
   long long gnbr_base;  // offset of group slot 0's row in the group-pair array
+  // entries a group-pair row holds: a quarter more than nbr_capacity, so that a build inside a block of
+  // steps that passes it loses no pair before the host looks
+  int gnbr_capacity;
   int grid[3];
   long long grid_base;  // real grid offset (K^3)
   long long half_base;  // complex half-spectrum offset (Kx*Ky*(Kz/2+1))

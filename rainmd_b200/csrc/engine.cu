@@ -176,6 +176,9 @@ static int grown_capacity(int capacity, int required) {
   return row_capacity(std::max(capacity + 32, (int)std::ceil(required * 1.25)));
 }
 
+// Entries a group-pair row holds (common.cuh DevSys::gnbr_capacity).
+static int group_row_capacity(int capacity) { return row_capacity(capacity + capacity / 4); }
+
 // How a force evaluation treats the neighbour lists.
 enum RebuildMode { REBUILD_NONE = 0, REBUILD_FORCED = 1, REBUILD_IF_STALE = 2 };
 
@@ -1292,7 +1295,8 @@ void Engine::allocate_neighbours() {
     total += (long long)hs[s].n * hs[s].capacity;
     const int groups = (s + 1 < S ? h_sys[s + 1].group_base : n_groups_total) - h_sys[s].group_base;
     h_sys[s].gnbr_base = group_total;
-    if (pair_list != 1) group_total += (long long)groups * hs[s].capacity;
+    h_sys[s].gnbr_capacity = group_row_capacity(hs[s].capacity);
+    if (pair_list != 1) group_total += (long long)groups * h_sys[s].gnbr_capacity;
   }
   // per-atom rows only where the pair loop or an inspection reads them
   nbr.alloc(pair_list == 0 ? 1 : total);
@@ -1316,6 +1320,7 @@ void Engine::allocate_neighbours() {
     cur[s].nbr_base = h_sys[s].nbr_base;
     cur[s].nbr_capacity = h_sys[s].nbr_capacity;
     cur[s].gnbr_base = h_sys[s].gnbr_base;
+    cur[s].gnbr_capacity = h_sys[s].gnbr_capacity;
   }
   CUDA_OK(cudaMemcpy(sys.p, cur.data(), sizeof(DevSys) * S, cudaMemcpyHostToDevice));
   h_sys = cur;
@@ -1733,7 +1738,7 @@ int Engine::check_capacity() {
     read_required();
     capacity_grew = true;
     for (int s = 0; s < S; ++s) {
-      if (req[s] > hs[s].capacity)
+      if (req[s] > (pair_list == 0 ? group_row_capacity(hs[s].capacity) : hs[s].capacity))
         throw Error(RMD_ERR_NEIGHBOUR_OVERFLOW,
                     "the neighbour list needed " + std::to_string(req[s]) + " slots per atom and the capacity is " +
                         std::to_string(hs[s].capacity) + ". Pairs were dropped, so the forces from this build are "
@@ -2749,7 +2754,7 @@ rmd_status rmd_debug_group_rows(rmd_sim *sim, int32_t s, int32_t *groups, int32_
     const auto &ds = e.h_sys[s];
     const int first = ds.group_base;
     const int n = (s + 1 < e.S ? e.h_sys[s + 1].group_base : e.n_groups_total) - first;
-    const int cap = ds.nbr_capacity;
+    const int cap = ds.gnbr_capacity;
     if (groups) *groups = n;
     if (capacity) *capacity = cap;
     if (!atoms && !counts && !partners) return;

@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(WARPS == 1 ? 128 : 32 * WARPS, WARPS == 8 ? 4 
   const int cc[3] = {cell0 / (counts[1] * counts[2]), (cell0 / counts[2]) % counts[1], cell0 % counts[2]};
   const bool rectangular = s.box[3] == 0.f && s.box[6] == 0.f && s.box[7] == 0.f;
   const float cull2 = s.list_cutoff2 * 1.00004f * 1.0001f;  // the margin k_neighbours culls with
-  const int cap = s.nbr_capacity;
+  const int cap = s.gnbr_capacity;
   int *row = gnbr + s.gnbr_base + (long long)q * cap;
   // visits an axis: its three stencil cells (each through its own wrap), or every cell of an axis of
   // fewer through each of three images

@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   // 46.7 -> 43.2, a batch of 24 124 -> 113)
   __shared__ float4 shift[4][32];
   const int wib = threadIdx.x >> 5;
-  const int *row = gnbr + s.gnbr_base + (long long)(warp - s.group_base) * s.nbr_capacity;
+  const int *row = gnbr + s.gnbr_base + (long long)(warp - s.group_base) * s.gnbr_capacity;
   // Rows too many for L2 are read from device memory: this one starts on its way while the records
   // below are read (250,000 atoms 354 -> 341 us; 99,999 143.0 -> 143.9 and a batch 112.6 -> 114, whose
   // rows stay in L2, hence the line).
