@@ -459,7 +459,11 @@ __device__ __forceinline__ void process_unit(const IntegrateArgs &g, int index, 
   const int sidx = g.sys_of_atom[u.atom[0]];
   res.sidx = sidx;
   const DevInteg p = g.integ[sidx];
+  const int local_base = g.sys_atom_start[sidx];
+  DevSettle sw;
+  if constexpr (KIND == 2) sw = g.settle_param[settle_index];
   SolverDiag dg = {0, 0, 0, 0.f};
+  chain_begin();  // (what is read above changes only between runs)
   if (MODE & INT_CONSTRAIN) {
     // minimiser: project the displaced positions back onto the constraints along the
     // pre-displacement geometry (encodeConstrainPositions, integrate.js:672-688)
@@ -476,7 +480,7 @@ __device__ __forceinline__ void process_unit(const IntegrateArgs &g, int index, 
     }
     if constexpr (KIND == 1) shake(u, cs, p, dg);
     if constexpr (KIND >= SHAPED) shake_shaped<SHAPE>(u, dist, p, dg);
-    if constexpr (KIND == 2) settle_positions(u, g.settle_param[settle_index], 1.0f);
+    if constexpr (KIND == 2) settle_positions(u, sw, 1.0f);
 #pragma unroll
     for (int k = 0; k < CAP; ++k) {
       if (k >= u.n) continue;
@@ -485,12 +489,24 @@ __device__ __forceinline__ void process_unit(const IntegrateArgs &g, int index, 
     }
     return;
   }
+  // Everything the unit reads, in one round trip: what the end of the step needs too (charge, wrap
+  // shift, displacement origin, slot), which used to be read after the constraints.
+  constexpr int KEEP = (MODE & INT_OPEN) && KIND != 1 ? CAP : 1;
+  float4 wrap[KEEP], start[KEEP];
+  float charge[KEEP];
+  int slot[KEEP];
 #pragma unroll
   for (int k = 0; k < CAP; ++k) {
     if (k >= u.n) continue;
     const int a = u.atom[k];
     const float4 x = g.posq[a];
     const float4 v = g.vel[a];
+    if ((MODE & INT_OPEN) && KIND != 1) {
+      wrap[k % KEEP] = g.wrap[a];
+      start[k % KEEP] = g.origin[a];
+      slot[k % KEEP] = g.rank[a];
+      charge[k % KEEP] = x.w;
+    }
     u.x[k][0] = x.x; u.x[k][1] = x.y; u.x[k][2] = x.z;
     u.v[k][0] = v.x; u.v[k][1] = v.y; u.v[k][2] = v.z;
     u.im[k] = v.w;  // inverse mass (0 for a massless site)
@@ -499,10 +515,7 @@ __device__ __forceinline__ void process_unit(const IntegrateArgs &g, int index, 
     u.f[k][2] = from_fixed(g.force[2 * (long long)g.n_atoms + a]);
   }
   const float h = p.half_step;
-  const int local_base = g.sys_atom_start[sidx];
   const uint32_t step = (uint32_t)(g.step_base[sidx] + g.step_offset);
-  DevSettle sw;
-  if constexpr (KIND == 2) sw = g.settle_param[settle_index];
   auto velocity_constraint = [&]() {
     if constexpr (KIND == 1) rattle(u, cs, p, dg);
     if constexpr (KIND >= SHAPED) rattle_shaped<SHAPE>(u, dist, p, dg);
@@ -551,12 +564,13 @@ __device__ __forceinline__ void process_unit(const IntegrateArgs &g, int index, 
     if (k >= u.n) continue;
     const int a = u.atom[k];
     if (MODE & INT_OPEN) {
-      const float4 old = g.posq[a];
-      g.posq[a] = make_float4(u.x[k][0], u.x[k][1], u.x[k][2], old.w);
+      const float q = KIND != 1 ? charge[k % KEEP] : g.posq[a].w;
+      g.posq[a] = make_float4(u.x[k][0], u.x[k][1], u.x[k][2], q);
       // keep the cell-ordered copy current: same wrap shift as at the last rebuild
-      const float4 w = g.wrap[a];
-      g.spos[g.rank[a]] = make_float4(u.x[k][0] - w.x, u.x[k][1] - w.y, u.x[k][2] - w.z, old.w);
-      const float4 o = g.origin[a];
+      const float4 w = KIND != 1 ? wrap[k % KEEP] : g.wrap[a];
+      g.spos[KIND != 1 ? slot[k % KEEP] : g.rank[a]] =
+          make_float4(u.x[k][0] - w.x, u.x[k][1] - w.y, u.x[k][2] - w.z, q);
+      const float4 o = KIND != 1 ? start[k % KEEP] : g.origin[a];
       const float dx = u.x[k][0] - o.x, dy = u.x[k][1] - o.y, dz = u.x[k][2] - o.z;
       worst = max(worst, __float_as_uint(dx * dx + dy * dy + dz * dz));
     }
@@ -568,7 +582,6 @@ __device__ __forceinline__ void process_unit(const IntegrateArgs &g, int index, 
 
 template <int MODE>
 __global__ void __launch_bounds__(64) k_integrate(IntegrateArgs g) {
-  chain_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool active = t < g.n_units;
@@ -583,6 +596,8 @@ __global__ void __launch_bounds__(64) k_integrate(IntegrateArgs g) {
     else if (k < g.shaped_end[2]) process_unit<MODE, SHAPED + 2, 3>(g, k, res);
     else if (k < g.shaped_end[3]) process_unit<MODE, SHAPED + 3, 4>(g, k, res);
     else process_unit<MODE, 2, 3>(g, k - g.shaped_end[3], res);
+  } else {
+    chain_begin();
   }
   if (MODE & INT_CONSTRAIN) return;  // every thread of the launch leaves here together
   // --- skin displacement and solver diagnostics, aggregated per warp when it is one system
