@@ -274,6 +274,7 @@ struct Engine {
   // trajectory output (traj.cu): per-molecule translations, a staging buffer, error slots
   DevArray<double3> traj_shift;
   DevArray<unsigned char> traj_out;
+  DevArray<float> state_out;  // readState's packed arrays
   DevArray<int> traj_status;
   TrajArgs traj_args(int s, bool image);  // sizes the scratch; computes the translations when imaging
   DevArray<double> mol_vir, e_term_vir;
@@ -293,6 +294,7 @@ struct Engine {
 
   ~Engine() {
     if (pinned) cudaFreeHost(pinned);
+    if (status_host) cudaFreeHost(status_host);
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -334,7 +336,18 @@ struct Engine {
   double tune_ms[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
   bool autotune();  // true when it launched timing work (the force array then holds its sums)
   void drop_graphs();
-  int check_capacity();  // returns max required; grows if needed
+  // the read-back block (allocate_status) and its host mirror
+  DevArray<unsigned char> status;
+  void *status_host = nullptr;
+  struct {
+    double *energies, *baro;
+    unsigned long long *builds;
+    int *required, *required_max;
+    unsigned *disp;
+  } seen{};
+  void allocate_status();
+  void read_status();
+  int check_capacity();  // from `seen`: returns max required; grows if needed
   bool capacity_grew = false;  // the last check_capacity grew the lists (and rebuilt them, forces only)
   void run(int64_t count, int block, const volatile int32_t *stop);
   void run_block(int n, bool barostat, bool energy_last);
@@ -997,10 +1010,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   e_acc.zero();
   rank.alloc(N);
   rank.zero();
-  required.alloc(2 * (size_t)S);  // longest per-atom row, then longest group-pair row, per system
-  required.zero();
-  required_max.alloc(S);
-  required_max.zero();
+  allocate_status();
   stale.alloc(S);
   stale.zero();
   saved_wrap.alloc(N);
@@ -1013,8 +1023,6 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   list_rebuilt.zero();
   spread_bits.alloc(S);
   spread_bits.zero();
-  list_builds.alloc(2);
-  list_builds.zero();
 
   // ---- PME grids, moduli, twiddles, FFT plans and task tables
   {
@@ -1178,12 +1186,8 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   integ.upload(h_integ);
   step_base.alloc(S);
   step_base.zero();
-  disp.alloc(2 * S);
-  disp.zero();
   diag.alloc(4 * S);
   diag.zero();
-  energies.alloc((size_t)S * N_ENERGY);
-  energies.zero();
   saved_energies.alloc((size_t)S * N_ENERGY);
   saved_energies.zero();
   fixed_scales.alloc(S);
@@ -1237,8 +1241,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
       if (o0.learned_steps_per_move > 0) learned_steps = o0.learned_steps_per_move;
       if (o0.learned_rate > 0) learned_lr = (float)o0.learned_rate;
     }
-    std::vector<double> tmp = hb;
-    baro.upload(tmp);
+    CUDA_OK(cudaMemcpy(baro.p, hb.data(), sizeof(double) * hb.size(), cudaMemcpyHostToDevice));
   }
   // ---- energy segments
   {
@@ -1285,6 +1288,43 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
     segments.upload(seg);
     seg_out.alloc(n_segments);
   }
+}
+
+// What the host reads back after a block of steps or an evaluation, in one allocation with a
+// page-locked mirror: one asynchronous copy and one wait, where each array had a copy and a wait of
+// its own (six after every block).
+void Engine::allocate_status() {
+  size_t bytes = 0;
+  auto place = [&](size_t n, size_t size) {
+    const size_t at = bytes;
+    bytes += (n * size + 15) / 16 * 16;
+    return at;
+  };
+  const size_t at_energies = place((size_t)S * N_ENERGY, sizeof(double)), at_baro = place((size_t)S * N_BARO, sizeof(double));
+  const size_t at_builds = place(2, sizeof(unsigned long long));
+  const size_t at_required = place(2 * (size_t)S, sizeof(int)), at_max = place(S, sizeof(int)),
+               at_disp = place(2 * (size_t)S, sizeof(unsigned));
+  status.alloc(bytes);
+  status.zero();
+  CUDA_OK(cudaMallocHost(&status_host, bytes));
+  memset(status_host, 0, bytes);
+  auto part = [&](auto &array, auto *&mirror, size_t at, size_t n) {
+    array.p = reinterpret_cast<decltype(array.p)>(status.p + at);  // (owned by `status`)
+    array.n = n;
+    mirror = reinterpret_cast<decltype(array.p)>(static_cast<char *>(status_host) + at);
+  };
+  part(energies, seen.energies, at_energies, (size_t)S * N_ENERGY);
+  part(baro, seen.baro, at_baro, (size_t)S * N_BARO);
+  part(list_builds, seen.builds, at_builds, 2);
+  part(required, seen.required, at_required, 2 * (size_t)S);  // longest per-atom row, then longest group-pair row, per system
+  part(required_max, seen.required_max, at_max, S);
+  part(disp, seen.disp, at_disp, 2 * (size_t)S);
+}
+
+// Bring `seen` up to date with everything queued on the stream.
+void Engine::read_status() {
+  CUDA_OK(cudaMemcpyAsync(status_host, status.p, status.n, cudaMemcpyDeviceToHost, stream));
+  sync();
 }
 
 void Engine::allocate_neighbours() {
@@ -1707,16 +1747,14 @@ void Engine::set_state(int s, const double *pos, const double *vel_in, int64_t s
 int Engine::check_capacity() {
   // the last build's requirement, and the largest of the builds before it since the last check;
   // the rows the pair loop walks are what diagnostics report
-  std::vector<int> req(S), earlier(S);
+  std::vector<int> req(S), earlier(seen.required_max, seen.required_max + S);
   auto read_required = [&]() {
-    std::vector<int> both(2 * (size_t)S);
-    CUDA_OK(cudaMemcpy(both.data(), required.p, sizeof(int) * both.size(), cudaMemcpyDeviceToHost));
-    for (int s = 0; s < S; ++s) req[s] = std::max(both[s], both[S + s]);
+    for (int s = 0; s < S; ++s) req[s] = std::max(seen.required[s], seen.required[S + s]);
   };
   read_required();
   capacity_grew = false;
-  CUDA_OK(cudaMemcpy(earlier.data(), required_max.p, sizeof(int) * S, cudaMemcpyDeviceToHost));
-  CUDA_OK(cudaMemset(required_max.p, 0, sizeof(int) * S));
+  if (std::any_of(earlier.begin(), earlier.end(), [](int v) { return v != 0; }))
+    CUDA_OK(cudaMemsetAsync(required_max.p, 0, sizeof(int) * S, stream));
   bool grow = false;
   int worst = 0;
   for (int s = 0; s < S; ++s) {
@@ -1733,8 +1771,8 @@ int Engine::check_capacity() {
   if (grow) {
     allocate_neighbours();
     evaluate(true, false);
-    sync();
-    CUDA_OK(cudaMemset(required_max.p, 0, sizeof(int) * S));
+    read_status();
+    CUDA_OK(cudaMemsetAsync(required_max.p, 0, sizeof(int) * S, stream));
     read_required();
     capacity_grew = true;
     for (int s = 0; s < S; ++s) {
@@ -1858,7 +1896,10 @@ bool Engine::autotune() {
 
 void Engine::initialise() {
   evaluate(true, false);
-  sync();
+  // kinetic energies of the current velocities, for energy() before any step
+  launch_integrate(iargs(0), INT_CLOSE_KINETIC, stream);
+  kernel_launches += 1;
+  read_status();
   for (auto &h : hs) h.steps_since_rebuild = 0;
   check_capacity();
   // the forces from a clean evaluation when the autotuner's timed pair-loop launches added into
@@ -1867,10 +1908,6 @@ void Engine::initialise() {
     evaluate(false, false);
     sync();
   }
-  // kinetic energies of the current velocities, for energy() before any step
-  launch_integrate(iargs(0), INT_CLOSE_KINETIC, stream);
-  kernel_launches += 1;
-  sync();
 }
 
 // The captured graph of a block of n steps (with a volume move first, and an energy-enabled
@@ -1960,11 +1997,9 @@ void Engine::run_block(int n, bool barostat, bool energy_last) {
 
 // #checkSkin (simulation.js:544-623) and #checkNeighbourCapacity (simulation.js:424-443)
 void Engine::check_block(int steps) {
-  std::vector<unsigned> d(2 * S);
-  CUDA_OK(cudaMemcpy(d.data(), disp.p, sizeof(unsigned) * 2 * S, cudaMemcpyDeviceToHost));
+  const unsigned *d = seen.disp;
   if (on_demand) {  // the rebuild bodies that ran inside the block's graph
-    unsigned long long taken = 0;
-    CUDA_OK(cudaMemcpy(&taken, list_builds.p, sizeof taken, cudaMemcpyDeviceToHost));
+    const unsigned long long taken = seen.builds[0];
     kernel_launches += (1LL + rebuild_launches(ctx())) * (long long)(taken - conditional_builds_seen);
     conditional_builds_seen = taken;
   }
@@ -2058,14 +2093,12 @@ void Engine::run(int64_t count, int block, const volatile int32_t *stop) {
       CUDA_OK(cudaEventElapsedTime(&ms, ev_a, ev_b));
       timed_ms += ms;
     }
-    sync();
+    read_status();
     if (due) {
       for (auto &h : hs) h.steps_since_barostat = 0;
-      std::vector<double> b((size_t)S * N_BARO);
-      CUDA_OK(cudaMemcpy(b.data(), baro.p, sizeof(double) * b.size(), cudaMemcpyDeviceToHost));
       for (int s = 0; s < S; ++s) {
         HostSystem &h = hs[s];
-        const double *bb = b.data() + (size_t)s * N_BARO;
+        const double *bb = seen.baro + (size_t)s * N_BARO;
         if (!h.has_pressure) continue;
         rmd_volume_move &m = h.last_move;
         m.attempted = 1;
@@ -2098,12 +2131,11 @@ void Engine::energy(int s, rmd_energy_report *out) {
   // forces and energies at the current positions, with the current list (no rebuild: the
   // skin keeps it valid), then the kinetic sums (simulation.js:1073-1230)
   evaluate(false, true);
-  sync();
-  const std::vector<double> all = read_energies();
-  const double *e = all.data() + (size_t)s * N_ENERGY;
+  DevSysD &d = *reinterpret_cast<DevSysD *>(staging(sizeof(DevSysD)));
+  CUDA_OK(cudaMemcpyAsync(&d, sysd.p + s, sizeof d, cudaMemcpyDeviceToHost, stream));
+  read_status();
+  const double *e = seen.energies + (size_t)s * N_ENERGY;
   HostSystem &h = hs[s];
-  DevSysD d;
-  CUDA_OK(cudaMemcpy(&d, sysd.p + s, sizeof d, cudaMemcpyDeviceToHost));
   memset(out, 0, sizeof *out);
   out->step = h.step;
   out->time = h.step * h.opt.timestep;
@@ -2202,7 +2234,7 @@ double Engine::scale_volume(int s, double ls) {
   CUDA_OK(cudaMemcpy(sysd.p + s, &d, sizeof d, cudaMemcpyHostToDevice));
   launch_update_box(sys.p, sysd.p, S, stream);
   evaluate(true, true);
-  sync();
+  read_status();
   for (auto &h : hs) h.steps_since_rebuild = 0;
   check_capacity();
   if (capacity_grew) {  // the first evaluation dropped pairs: its energy is not the potential
@@ -2242,7 +2274,7 @@ void Engine::minimise(int max_iterations, double force_tolerance, double max_ste
   if (!(cap > 0)) cap = 0.05;
   auto potentials = [&]() {
     evaluate(true, true);
-    sync();
+    read_status();
     for (auto &h : hs) h.steps_since_rebuild = 0;
     check_capacity();
     std::vector<double> e = read_energies(), p(S);
@@ -2563,38 +2595,30 @@ rmd_status rmd_read_state_at(rmd_sim *sim, int32_t s, float *positions, float *v
   return guarded(sim, [&]() {
     auto &e = sim->engine;
     const auto &h = e.hs[s];
-    // every requested array in one round of asynchronous copies into page-locked staging
+    // the requested arrays, packed on the device as the caller holds them (3 floats an atom), in one
+    // asynchronous copy into page-locked staging
     e.sync();
     const size_t n = (size_t)h.n;
-    char *stage = e.staging(sizeof(float4) * 2 * n + sizeof(long long) * 3 * n + sizeof(rmd::DevSysD));
-    float4 *p = reinterpret_cast<float4 *>(stage), *v = p + n;
-    long long *f = reinterpret_cast<long long *>(v + n);
-    rmd::DevSysD *d = reinterpret_cast<rmd::DevSysD *>(f + 3 * n);
-    if (positions)
-      CUDA_OK(cudaMemcpyAsync(p, e.posq.p + h.atom_start, sizeof(float4) * n, cudaMemcpyDeviceToHost, e.stream));
-    if (velocities)
-      CUDA_OK(cudaMemcpyAsync(v, e.vel.p + h.atom_start, sizeof(float4) * n, cudaMemcpyDeviceToHost, e.stream));
-    if (forces)
-      for (int c = 0; c < 3; ++c)
-        CUDA_OK(cudaMemcpyAsync(f + c * n, e.force.p + (size_t)c * e.N + h.atom_start, sizeof(long long) * n,
-                                cudaMemcpyDeviceToHost, e.stream));
+    const int parts = (positions ? 1 : 0) + (velocities ? 1 : 0) + (forces ? 1 : 0);
+    char *stage = e.staging(sizeof(float) * 3 * n * parts + sizeof(rmd::DevSysD));
+    rmd::DevSysD *d = reinterpret_cast<rmd::DevSysD *>(stage);
+    float *packed = reinterpret_cast<float *>(stage + sizeof(rmd::DevSysD));
+    if (parts) {
+      if (e.state_out.n < 3 * n * parts) e.state_out.alloc(3 * n * parts);
+      rmd::launch_pack_state(e.posq.p + h.atom_start, e.vel.p + h.atom_start, e.force.p + h.atom_start, e.N, h.n,
+                             positions != nullptr, velocities != nullptr, forces != nullptr, e.state_out.p, e.stream);
+      e.kernel_launches += 1;
+      CUDA_OK(cudaGetLastError());
+      CUDA_OK(cudaMemcpyAsync(packed, e.state_out.p, sizeof(float) * 3 * n * parts, cudaMemcpyDeviceToHost, e.stream));
+    }
     if (box_vectors || volume)
       CUDA_OK(cudaMemcpyAsync(d, e.sysd.p + s, sizeof(rmd::DevSysD), cudaMemcpyDeviceToHost, e.stream));
     e.sync();
-    for (size_t i = 0; i < n; ++i) {
-      if (positions) {
-        positions[3 * i] = p[i].x;
-        positions[3 * i + 1] = p[i].y;
-        positions[3 * i + 2] = p[i].z;
+    for (float *out : {positions, velocities, forces})
+      if (out) {
+        memcpy(out, packed, sizeof(float) * 3 * n);
+        packed += 3 * n;
       }
-      if (velocities) {
-        velocities[3 * i] = v[i].x;
-        velocities[3 * i + 1] = v[i].y;
-        velocities[3 * i + 2] = v[i].z;
-      }
-      if (forces)
-        for (int c = 0; c < 3; ++c) forces[3 * i + c] = (float)((double)f[c * n + i] / rmd::FORCE_SCALE);
-    }
     if (box_vectors)
       for (int k = 0; k < 9; ++k) box_vectors[k] = d->box[k];
     if (volume) *volume = d->volume;
@@ -2788,7 +2812,7 @@ rmd_status rmd_debug_evaluate(rmd_sim *sim, int32_t s, rmd_energy_report *energy
   return guarded(sim, [&]() {
     auto &e = sim->engine;
     e.evaluate(true, true);
-    e.sync();
+    e.read_status();
     for (auto &h : e.hs) h.steps_since_rebuild = 0;
     e.check_capacity();
     e.energy(s, energy);

@@ -366,6 +366,10 @@ struct Rst7Box {
   double values[6];      // lengths in angstroms, angles in degrees
   double velocity_unit;  // nm/ps per angstrom per AMBER time unit
 };
+// Positions, velocities and forces (those asked for, in this order) of n atoms as 3 floats an atom;
+// `force` is the first of the atoms' x components in the [3][n_total] fixed-point array.
+void launch_pack_state(const float4 *posq, const float4 *vel, const unsigned long long *force, int n_total, int n,
+                       bool positions, bool velocities, bool forces, float *out, cudaStream_t stream);
 void launch_traj_shifts(const TrajArgs &t, cudaStream_t stream);
 void launch_traj_image(const TrajArgs &t, double *out, cudaStream_t stream);
 void launch_dcd_pack(const TrajArgs &t, int periodic, cudaStream_t stream);
