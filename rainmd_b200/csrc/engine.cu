@@ -2322,7 +2322,12 @@ void Engine::minimise(int max_iterations, double force_tolerance, double max_ste
   const long long limit = (long long)(max_iterations + 1) * (MIN_ATTEMPTS + 1) + 64;
   long long trials = 0;
   while (trials < limit) {
-    const int batch = (int)std::min<long long>(16, limit - trials);
+    // trials past the last one are launched in vain (each evaluates its forces all the same), so few
+    // at a time when few iterations are left: every open iteration takes at least one
+    int left = 0;
+    for (int s = 0; s < S; ++s)
+      if (!state[s].done) left = std::max(left, max_iterations - state[s].iterations);
+    const int batch = (int)std::min<long long>(left >= 32 ? 16 : std::max(2, std::min(8, left)), limit - trials);
     for (int k = 0; k < batch; ++k) CUDA_OK(cudaGraphLaunch(trial, stream));
     trials += batch;
     kernel_launches += trial_kernels * batch;
@@ -2361,10 +2366,7 @@ void Engine::minimise(int max_iterations, double force_tolerance, double max_ste
   // forces at the final structure, and velocities zeroed (simulation.js:971-973)
   const std::vector<double> potential = potentials();
   std::vector<float> worst = max_forces();
-  std::vector<float4> v(N);
-  CUDA_OK(cudaMemcpy(v.data(), vel.p, sizeof(float4) * N, cudaMemcpyDeviceToHost));
-  for (auto &x : v) x.x = x.y = x.z = 0.f;
-  CUDA_OK(cudaMemcpy(vel.p, v.data(), sizeof(float4) * N, cudaMemcpyHostToDevice));
+  CUDA_OK(cudaMemset2DAsync(vel.p, sizeof(float4), 0, 3 * sizeof(float), N, stream));  // (w: the inverse mass)
   launch_integrate(iargs(0), INT_CLOSE_KINETIC, stream);
   sync();
   if (out) {
