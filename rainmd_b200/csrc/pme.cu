@@ -817,13 +817,12 @@ static void launch_gather(const LaunchCtx &c, cudaStream_t stream) {
 
 // Forward transform of the spread grid to the half spectrum (z and y; x is left to the caller).
 static void launch_forward_zy(const LaunchCtx &c, cudaStream_t stream, bool all = false) {
-  // A plain launch: the first FFT pass waits for the spreading's last atomics like any kernel
-  // boundary. Chained after the spreading it was slower on one B200 at 64^3 (the seven
-  // reciprocal kernels 0.067 against 0.049 ms, the 23,558-atom step 0.1394 against 0.1358 ms)
-  // and no faster at 32^3 or 100^3. It still lets the next pass be scheduled early.
+  // The two-factor pass is chained after the spreading like the rest (it reads its tables while the
+  // last atomics land: the reciprocal kernels 33.1 -> 30.8 us at 64^3, 20.5 -> 17.9 at 24^3). The
+  // generic pass stays a plain launch: chained it was slower at 64^3 (0.067 against 0.049 ms).
   if (c.n_tasks_z2 > 0)
-    (c.fft_large ? k_fft_r2c<RADIX_ALL> : k_fft_r2c<RADIX_SMALL>)<<<c.n_tasks_z2, c.z2_threads, c.z2_smem * sizeof(float2), stream>>>(
-        c.tasks_z2, c.twiddles, c.fixed_grid, c.half);
+    launch_kernel(c.chain_pme, c.fft_large ? k_fft_r2c<RADIX_ALL> : k_fft_r2c<RADIX_SMALL>, c.n_tasks_z2, c.z2_threads,
+                  c.z2_smem * sizeof(float2), stream, c.tasks_z2, c.twiddles, c.fixed_grid, c.half);
   if (c.n_tasks_z > 0)
     k_fft_z_r2c<<<c.n_tasks_z, 256, 0, stream>>>(c.tasks_z, c.sys, c.fft_plans, c.twiddles, c.fixed_grid, c.half);
   const FftTask *ty = all ? c.tasks_y_all : c.tasks_y;
