@@ -217,16 +217,26 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
   int *slice = cell_atoms + s.atom_start + begin;
   const int gbase = s.atom_start + begin;
   constexpr int SMEM = 2048;
-  __shared__ int keys[SMEM];
-  __shared__ int sub_keys[SMEM];
+  __shared__ __align__(16) int keys[SMEM + 4];
+  __shared__ __align__(16) int sub_keys[SMEM + 4];
   __shared__ int sorted[SMEM];
+  // how many of the n values (padded with INT_MAX to a multiple of 4) are below `key`: all pairs, four
+  // to a shared-memory read
+  auto below = [&](const int *values, int key) {
+    int rank = 0;
+    for (int m = 0; m < n; m += 4) {
+      const int4 k4 = *reinterpret_cast<const int4 *>(values + m);
+      rank += (k4.x < key) + (k4.y < key) + (k4.z < key) + (k4.w < key);
+    }
+    return rank;
+  };
   const bool by_group = v.group_box != nullptr;
   if (n <= SMEM) {
     for (int k = threadIdx.x; k < n; k += blockDim.x) keys[k] = slice[k];
+    if (threadIdx.x < 4) keys[n + threadIdx.x] = sub_keys[n + threadIdx.x] = INT_MAX;
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      int key = keys[k], rank = 0;
-      for (int m = 0; m < n; ++m) rank += keys[m] < key;
+      const int key = keys[k], rank = below(keys, key);
       slice[rank] = key;
       if (by_group) {
         float fl[3];
@@ -238,8 +248,7 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
     }
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      int key = sub_keys[k], rank = 0;
-      for (int m = 0; m < n; ++m) rank += sub_keys[m] < key;
+      const int rank = below(sub_keys, sub_keys[k]);
       if (by_group) {
         place_sorted(v, s, gbase + rank, sorted[k], cc);
         v.group_order[gbase + k] = gbase + k;
