@@ -121,8 +121,8 @@ typedef struct {
    * simulation.js:544-623). No reference counterpart. */
   int32_t rebuild_on_demand;
   /* Which neighbour structure the pair loop walks. 0 (default): per 4-atom group of
-   * spatially close atoms, the half list of partner atoms within cutoff + skin of the group's
-   * bounding box, each pair evaluated once and its force added to both atoms (64-bit
+   * spatially close atoms, the half list of partner atoms within cutoff + skin of one of the
+   * four, each pair evaluated once and its force added to both atoms (64-bit
    * fixed-point atomics for the partner); needs force_accumulation 0 and at most 2^23 atoms
    * in the handle, else 1 is used. 1: the reference's full per-atom rows (neighbours.js:46-151),
    * each pair evaluated from both atoms. 2: as 0, and every build also writes the per-atom

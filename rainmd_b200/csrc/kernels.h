@@ -134,7 +134,7 @@ struct LaunchCtx {
   // build also writes the per-atom rows (rmd_options.pair_list)
   int pair_list;
   int *gnbr, *gnbr_count;  // group-pair rows and their lengths, per group slot
-  int *gfirst, *gsize;     // per group slot: its first position in group_order, its atoms (0: unused)
+  int *gfirst, *gsize;     // per group slot: its first slot, its atoms (0: unused)
   int2 *slot_info;         // per slot: LJ type, original index
   int *group_cell;         // per group slot: its cell
   float4 *group_box;       // per group slot: bounding box lo, hi of its atoms' wrapped positions
