@@ -188,8 +188,8 @@ struct Engine {
   cudaStream_t stream = nullptr;
   // the reciprocal-space branch of a force evaluation runs on `side`, forked from and joined
   // back to `stream` with events (inside a captured graph these become parallel branches)
-  cudaStream_t side = nullptr, bonded = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_clear = nullptr, ev_bonded = nullptr;
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_clear = nullptr;
   // the stream a conditional rebuild body is captured on (record_forces)
   cudaStream_t cond = nullptr;
   bool on_demand = true;  // lists rebuilt when the device finds them stale (all systems agree)
@@ -299,8 +299,6 @@ struct Engine {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_clear) cudaEventDestroy(ev_clear);
-    if (ev_bonded) cudaEventDestroy(ev_bonded);
-    if (bonded) cudaStreamDestroy(bonded);
     if (side) cudaStreamDestroy(side);
     if (cond) cudaStreamDestroy(cond);
     if (stream) cudaStreamDestroy(stream);
@@ -584,14 +582,12 @@ void Engine::build(int count, const rmd_system *systems, const rmd_options *opti
   // giving them the highest priority (cudaGraphInstantiateFlagUseNodePriority) slowed the NVT
   // step from 0.101 to 0.104 ms, and the pair branch the higher one changed nothing.
   CUDA_OK(cudaStreamCreateWithFlags(&side, cudaStreamDefault));
-  CUDA_OK(cudaStreamCreateWithFlags(&bonded, cudaStreamDefault));
   CUDA_OK(cudaStreamCreateWithFlags(&cond, cudaStreamNonBlocking));
   on_demand = true;
   for (auto &h : hs) on_demand = on_demand && h.on_demand;
   CUDA_OK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
   CUDA_OK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
   CUDA_OK(cudaEventCreateWithFlags(&ev_clear, cudaEventDisableTiming));
-  CUDA_OK(cudaEventCreateWithFlags(&ev_bonded, cudaEventDisableTiming));
   upload_all(src);
 }
 
@@ -1630,16 +1626,8 @@ void Engine::record_forces(int rebuild, bool energy) {
     launch_pme_gather(c, side);
     CUDA_OK(cudaEventRecord(ev_join, side));
   }
-  // so does the bonded kernel, on a branch of its own beside the pair kernel
-  const bool bonded_beside = gather_beside && n_bonds + n_angles + n_tors + n_rest > 0;
-  if (bonded_beside) {
-    CUDA_OK(cudaStreamWaitEvent(bonded, ev_clear, 0));
-    launch_bonded(c, energy, bonded);
-    CUDA_OK(cudaEventRecord(ev_bonded, bonded));
-  }
   launch_nonbonded(nb, energy, nb_lanes, stream);
-  if (bonded_beside) CUDA_OK(cudaStreamWaitEvent(stream, ev_bonded, 0));
-  else launch_bonded(c, energy, stream);
+  launch_bonded(c, energy, stream);
   if (pme_on) {
     CUDA_OK(cudaStreamWaitEvent(stream, ev_join, 0));
     if (!gather_beside) launch_pme_gather(c, stream);
