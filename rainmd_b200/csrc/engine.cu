@@ -270,7 +270,8 @@ struct Engine {
   DevArray<int3> settle_atoms;
   DevArray<DevSettle> settle_param;
   int n_free = 0, n_clusters = 0, n_settle = 0;
-  DevArray<int> mol_start, mol_atoms, mol_of_atom;
+  DevArray<int> mol_start, mol_atoms, mol_of_atom, mol_large;
+  int n_mol_large = 0;
   // trajectory output (traj.cu): per-molecule translations, a staging buffer, error slots
   DevArray<double3> traj_shift;
   DevArray<unsigned char> traj_out;
@@ -934,6 +935,12 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
     mol_start.upload(ms);
     mol_atoms.upload(ma);
     mol_of_atom.upload(moa);
+    std::vector<int> large;
+    for (int m = 0; m < n_molecules_total; ++m)
+      if (ms[m + 1] - ms[m] > SMALL_MOLECULE) large.push_back(m);
+    n_mol_large = (int)large.size();
+    if (large.empty()) large.push_back(0);
+    mol_large.upload(large);
   }
 
   // ---- cells
@@ -1440,6 +1447,8 @@ LaunchCtx Engine::ctx() const {
   c.masses = masses.p;
   c.mol_vir = mol_vir.p;
   c.n_molecules = n_molecules_total;
+  c.mol_large = mol_large.p;
+  c.n_mol_large = n_mol_large;
   c.pme_on = pme_on ? 1 : 0;
   c.pme_order = pme_order;
   c.fixed_grid = fixed_grid.p;
@@ -1562,6 +1571,8 @@ BaroArgs Engine::bargs() const {
   a.n_systems = S;
   a.n_atoms = N;
   a.n_molecules = n_molecules_total;
+  a.mol_large = mol_large.p;
+  a.n_mol_large = n_mol_large;
   a.posq = posq.p;
   a.saved_posq = saved_posq.p;
   a.force = force.p;

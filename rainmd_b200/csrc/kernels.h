@@ -79,6 +79,16 @@ enum IntegrateMode {
   INT_CONSTRAIN = 16     // positions only: SHAKE/SETTLE towards saved_posq (minimiser)
 };
 
+// Kernels over molecules: the first blocks take a molecule of up to SMALL_MOLECULE atoms a thread, the
+// rest a larger one a warp.
+constexpr int SMALL_MOLECULE = 8, MOLECULE_THREADS = 128;
+__host__ __device__ constexpr int small_molecule_blocks(int n_molecules) {
+  return (n_molecules + MOLECULE_THREADS - 1) / MOLECULE_THREADS;
+}
+constexpr int molecule_blocks(int n_molecules, int n_large) {
+  return small_molecule_blocks(n_molecules) + (int)((32LL * n_large + MOLECULE_THREADS - 1) / MOLECULE_THREADS);
+}
+
 struct IntegrateArgs {
   int n_units, n_free, n_clusters, n_settle, n_atoms, n_systems;
   const int *free_atoms;
@@ -155,6 +165,8 @@ struct LaunchCtx {
   double *e_lj, *e_coul, *e_vir;
   // molecules, for the molecular virial correction (energy evaluations only)
   const int *mol_start, *mol_atoms;
+  const int *mol_large;  // the molecules of more than SMALL_MOLECULE atoms
+  int n_mol_large;
   const float *masses;
   double *mol_vir;
   int n_molecules;
@@ -275,6 +287,8 @@ struct BaroArgs {
   float4 *saved_posq;
   unsigned long long *force, *saved_force;
   const int *mol_start, *mol_atoms, *mol_of_atom;
+  const int *mol_large;  // the molecules of more than SMALL_MOLECULE atoms
+  int n_mol_large;
   const int *sys_of_atom;
   float4 *centroid;  // per molecule
   DevSys *sys;

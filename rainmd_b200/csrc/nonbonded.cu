@@ -768,10 +768,10 @@ void launch_bonded(const LaunchCtx &c, bool energy, cudaStream_t stream) {
 // After every force term: sum_i F_i.(r_i - R) over each molecule's atoms, R its centre of mass
 // (positions are never wrapped, so molecules are whole). Added to the atomic virial it turns
 // dU/dlnV for atoms scaled with the box into dU/dlnV for molecules scaled rigidly about their
-// centres. A molecule of up to SMALL_MOLECULE atoms is one thread's, the larger ones among a
-// warp's 32 are taken by the whole warp in turn: a warp for every molecule, 29 of 32 lanes idle on
-// water, took 51 us at 250,000 atoms, this 19 us.
-constexpr int SMALL_MOLECULE = 8;
+// centres. A molecule of up to SMALL_MOLECULE atoms is one thread's, a larger one a warp's: a warp for
+// every molecule, 29 of 32 lanes idle on water, took 51 us at 250,000 atoms, this 19 us. (The larger ones among
+// 32 walked in turn by the warp that holds them are a chain of up to 32 molecules: an energy report of 99,999
+// atoms in molecules of 1,200 then took 1,269 us, against 322 with a warp each.)
 template <int WIDTH>
 __device__ __forceinline__ double molecule_virial(const float4 *__restrict__ posq, const float *__restrict__ masses,
                                                   const int *__restrict__ mol_atoms,
@@ -813,24 +813,27 @@ __device__ __forceinline__ double molecule_virial(const float4 *__restrict__ pos
 __global__ void k_molecular_virial(const float4 *__restrict__ posq, const float *__restrict__ masses,
                                    const int *__restrict__ mol_start, const int *__restrict__ mol_atoms,
                                    const unsigned long long *__restrict__ force, double *__restrict__ mol_vir,
-                                   int n_molecules, int n_atoms) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-  const int begin = m < n_molecules ? mol_start[m] : 0, end = m < n_molecules ? mol_start[m + 1] : 0;
-  if (m < n_molecules && end - begin <= SMALL_MOLECULE)
-    mol_vir[m] = end > begin ? molecule_virial<1>(posq, masses, mol_atoms, force, begin, end, 0, n_atoms) : 0.0;
-  for (unsigned large = __ballot_sync(0xffffffffu, end - begin > SMALL_MOLECULE); large; large &= large - 1u) {
-    const int from = __ffs(large) - 1;
-    const double v = molecule_virial<32>(posq, masses, mol_atoms, force, __shfl_sync(0xffffffffu, begin, from),
-                                         __shfl_sync(0xffffffffu, end, from), lane, n_atoms);
-    if (lane == from) mol_vir[m] = v;
+                                   const int *__restrict__ mol_large, int n_molecules, int n_large, int n_atoms) {
+  if (blockIdx.x < small_molecule_blocks(n_molecules)) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= n_molecules) return;
+    const int begin = mol_start[m], end = mol_start[m + 1];
+    if (end - begin <= SMALL_MOLECULE)
+      mol_vir[m] = end > begin ? molecule_virial<1>(posq, masses, mol_atoms, force, begin, end, 0, n_atoms) : 0.0;
+    return;
   }
+  const int w = ((blockIdx.x - small_molecule_blocks(n_molecules)) * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= n_large) return;
+  const int m = mol_large[w];
+  const double v = molecule_virial<32>(posq, masses, mol_atoms, force, mol_start[m], mol_start[m + 1], lane, n_atoms);
+  if (lane == 0) mol_vir[m] = v;
 }
 
 void launch_molecular_virial(const LaunchCtx &c, cudaStream_t stream) {
   if (c.n_molecules <= 0) return;
-  const int tb = 128;
-  k_molecular_virial<<<(c.n_molecules + tb - 1) / tb, tb, 0, stream>>>(c.posq, c.masses, c.mol_start, c.mol_atoms,
-                                                                       c.force, c.mol_vir, c.n_molecules, c.n_atoms);
+  k_molecular_virial<<<molecule_blocks(c.n_molecules, c.n_mol_large), MOLECULE_THREADS, 0, stream>>>(
+      c.posq, c.masses, c.mol_start, c.mol_atoms, c.force, c.mol_vir, c.mol_large, c.n_molecules, c.n_mol_large,
+      c.n_atoms);
 }
 
 }  // namespace rmd

@@ -285,17 +285,20 @@ __device__ __forceinline__ void centroid_scale(const BaroArgs &a, const double *
   }
 }
 
-// A molecule of up to SMALL_MOLECULE atoms is one thread's; the larger ones among a warp's 32 are
-// taken by the whole warp in turn (a warp for every molecule left 29 of 32 lanes idle on water).
-constexpr int SMALL_MOLECULE = 8;
+// A molecule of up to SMALL_MOLECULE atoms is one thread's, a larger one a warp's (a warp for every
+// molecule left 29 of 32 lanes idle on water).
 __global__ void k_baro_centroid_scale(BaroArgs a, int n_molecules, const double *__restrict__ fixed_scales) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-  const int begin = m < n_molecules ? a.mol_start[m] : 0, end = m < n_molecules ? a.mol_start[m + 1] : 0;
-  if (end > begin && end - begin <= SMALL_MOLECULE) centroid_scale<1>(a, fixed_scales, begin, end, 0);
-  for (unsigned large = __ballot_sync(0xffffffffu, end - begin > SMALL_MOLECULE); large; large &= large - 1u) {
-    const int from = __ffs(large) - 1;
-    centroid_scale<32>(a, fixed_scales, __shfl_sync(0xffffffffu, begin, from), __shfl_sync(0xffffffffu, end, from), lane);
+  if (blockIdx.x < small_molecule_blocks(n_molecules)) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= n_molecules) return;
+    const int begin = a.mol_start[m], end = a.mol_start[m + 1];
+    if (end > begin && end - begin <= SMALL_MOLECULE) centroid_scale<1>(a, fixed_scales, begin, end, 0);
+    return;
   }
+  const int w = ((blockIdx.x - small_molecule_blocks(n_molecules)) * blockDim.x + threadIdx.x) >> 5;
+  if (w >= a.n_mol_large) return;
+  const int m = a.mol_large[w];
+  centroid_scale<32>(a, fixed_scales, a.mol_start[m], a.mol_start[m + 1], threadIdx.x & 31);
 }
 
 // One thread per system moving on its current lists: the move changes a pair's vector by
@@ -406,12 +409,12 @@ void launch_baro_propose(const BaroArgs &a, cudaStream_t stream) {
   k_baro_propose<<<(a.n_systems + 63) / 64, 64, 0, stream>>>(a);
 }
 void launch_baro_scale(const BaroArgs &a, cudaStream_t stream) {
-  const int tb = 128;
-  k_baro_centroid_scale<<<(a.n_molecules + tb - 1) / tb, tb, 0, stream>>>(a, a.n_molecules, nullptr);
+  k_baro_centroid_scale<<<molecule_blocks(a.n_molecules, a.n_mol_large), MOLECULE_THREADS, 0, stream>>>(a, a.n_molecules,
+                                                                                                    nullptr);
 }
 void launch_scale_fixed(const BaroArgs &a, const double *scales, cudaStream_t stream) {
-  const int tb = 128;
-  k_baro_centroid_scale<<<(a.n_molecules + tb - 1) / tb, tb, 0, stream>>>(a, a.n_molecules, scales);
+  k_baro_centroid_scale<<<molecule_blocks(a.n_molecules, a.n_mol_large), MOLECULE_THREADS, 0, stream>>>(a, a.n_molecules,
+                                                                                                    scales);
 }
 void launch_baro_allow(const BaroArgs &a, cudaStream_t stream) {
   k_baro_allow<<<(a.n_systems + 63) / 64, 64, 0, stream>>>(a);
