@@ -46,8 +46,8 @@ struct DevArray {
   size_t n = 0;
   void alloc(size_t count) {
     release();
-    n = count;
     if (count) CUDA_OK(cudaMalloc(&p, sizeof(T) * count));
+    n = count;  // (nothing to use when the allocation failed)
   }
   void upload(const std::vector<T> &v) {
     alloc(v.size());
@@ -275,7 +275,7 @@ struct Engine {
   // trajectory output (traj.cu): per-molecule translations, a staging buffer, error slots
   DevArray<double3> traj_shift;
   DevArray<unsigned char> traj_out;
-  DevArray<float> state_out;  // readState's packed arrays
+  DevArray<float> state_out;  // readState's packed arrays, of the largest system
   DevArray<int> traj_status;
   TrajArgs traj_args(int s, bool image);  // sizes the scratch; computes the translations when imaging
   DevArray<double> mol_vir, e_term_vir;
@@ -1017,6 +1017,9 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   e_acc.zero();
   rank.alloc(N);
   rank.zero();
+  int largest = 0;
+  for (auto &h : hs) largest = std::max(largest, h.n);
+  state_out.alloc(9 * (size_t)largest);
   allocate_status();
   stale.alloc(S);
   stale.zero();
@@ -2617,7 +2620,6 @@ rmd_status rmd_read_state_at(rmd_sim *sim, int32_t s, float *positions, float *v
     rmd::DevSysD *d = reinterpret_cast<rmd::DevSysD *>(stage);
     float *packed = reinterpret_cast<float *>(stage + sizeof(rmd::DevSysD));
     if (parts) {
-      if (e.state_out.n < 3 * n * parts) e.state_out.alloc(3 * n * parts);
       rmd::launch_pack_state(e.posq.p + h.atom_start, e.vel.p + h.atom_start, e.force.p + h.atom_start, e.N, h.n,
                              positions != nullptr, velocities != nullptr, forces != nullptr, e.state_out.p, e.stream);
       e.kernel_launches += 1;
