@@ -44,6 +44,11 @@ template <class T>
 struct DevArray {
   T *p = nullptr;
   size_t n = 0;
+  bool owned = true;  // false: a part of another array
+  DevArray() = default;
+  DevArray(const DevArray &) = delete;
+  DevArray &operator=(const DevArray &) = delete;
+  ~DevArray() { release(); }
   void alloc(size_t count) {
     release();
     if (count) CUDA_OK(cudaMalloc(&p, sizeof(T) * count));
@@ -56,10 +61,17 @@ struct DevArray {
   void zero() {
     if (n) CUDA_OK(cudaMemset(p, 0, sizeof(T) * n));
   }
+  void view(T *at, size_t count) {
+    release();
+    p = at;
+    n = count;
+    owned = false;
+  }
   void release() {
-    if (p) cudaFree(p);
+    if (p && owned) cudaFree(p);
     p = nullptr;
     n = 0;
+    owned = true;
   }
   size_t bytes() const { return sizeof(T) * n; }
 };
@@ -297,6 +309,8 @@ struct Engine {
     if (pinned) cudaFreeHost(pinned);
     if (status_host) cudaFreeHost(status_host);
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+    for (cudaEvent_t ev : {ev_a, ev_b})
+      if (ev) cudaEventDestroy(ev);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_clear) cudaEventDestroy(ev_clear);
@@ -1319,8 +1333,7 @@ void Engine::allocate_status() {
   CUDA_OK(cudaMallocHost(&status_host, bytes));
   memset(status_host, 0, bytes);
   auto part = [&](auto &array, auto *&mirror, size_t at, size_t n) {
-    array.p = reinterpret_cast<decltype(array.p)>(status.p + at);  // (owned by `status`)
-    array.n = n;
+    array.view(reinterpret_cast<decltype(array.p)>(status.p + at), n);
     mirror = reinterpret_cast<decltype(array.p)>(static_cast<char *>(status_host) + at);
   };
   part(energies, seen.energies, at_energies, (size_t)S * N_ENERGY);
