@@ -7,6 +7,7 @@
 // the on-device barostat can change it inside a CUDA graph.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -48,9 +49,12 @@ struct DevSys {
   // entries a group-pair row holds: a quarter more than nbr_capacity, so that a build inside a block of
   // steps that passes it loses no pair before the host looks
   int gnbr_capacity;
-  int grid[3];
+  // Never written after the engine is built, and read by the spreading before it waits for its predecessor
+  // (chain_begin): in a memory line that holds nothing else, because a line that such a read brings into a cache
+  // stays as it was when the volume move's kernels write the box.
+  alignas(128) int grid[3];
   long long grid_base;  // real grid offset (K^3)
-  long long half_base;  // complex half-spectrum offset (Kx*Ky*(Kz/2+1))
+  alignas(128) long long half_base;  // complex half-spectrum offset (Kx*Ky*(Kz/2+1))
   int moduli_base;      // moduli[x][y][z] concatenated (Kx+Ky+Kz)
   int order;
   int molecule_start, molecule_count;  // into molecule CSR
@@ -59,6 +63,9 @@ struct DevSys {
   // its partner that was nearest when the list was built (d = x_i - x_j - S).
   float4 shift[27];
 };
+static_assert(sizeof(DevSys) % 128 == 0 && offsetof(DevSys, grid) % 128 == 0 && offsetof(DevSys, half_base) % 128 == 0 &&
+                  offsetof(DevSys, half_base) - offsetof(DevSys, grid) == 128,
+              "the fields read before chain_begin() share no line with the others");
 
 // FP64 per-system state owned by the device (box for the barostat, energies, counters).
 struct DevSysD {
@@ -80,9 +87,11 @@ struct DevSysD {
 // The kernels of the step's serial chains (integrator, spreading, FFT passes, gather) are
 // launched with programmatic stream serialisation (launch_chained): a kernel's blocks may be
 // scheduled while its predecessor in the stream is still running, which hides the launch
-// latency between short dependent kernels. Such a kernel must start with chain_begin(): it
-// waits until every predecessor grid has completed and its memory is visible, before any
-// memory access, then lets its own successor be scheduled. In a plain launch both are no-ops.
+// latency between short dependent kernels. Every thread of such a kernel calls chain_begin(): it
+// waits until every predecessor grid has completed and its memory is visible, then lets the
+// kernel's own successor be scheduled. Before it a kernel writes nothing, and reads only what no kernel of
+// the engine writes: tables made with the handle (index lists, FFT tasks, twiddles, moduli), DevInteg, which
+// set_state alone writes, between launches, and of DevSys grid and grid_base. In a plain launch both are no-ops.
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

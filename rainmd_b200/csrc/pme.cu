@@ -139,7 +139,7 @@ __global__ void k_spread(const float4 *__restrict__ posq, const int *__restrict_
   const DevSys &s = sys[valid ? sys_of_atom[i] : 0];
   const int nx = s.grid[0], ny = s.grid[1], nz = s.grid[2];
   unsigned long long *grid = fixed_grid + s.grid_base;
-  chain_begin();  // (the system's grid never changes; positions and box do)
+  chain_begin();  // (DevSys::grid and grid_base never change; positions and box do)
   if (!valid) return;
   const int ky = (int)(t % (ORDER * ORDER)) / ORDER, kz = (int)(t % ORDER);
   const float4 p = posq[i];
