@@ -1803,7 +1803,7 @@ int Engine::check_capacity() {
     read_required();
     capacity_grew = true;
     for (int s = 0; s < S; ++s) {
-      if (req[s] > (pair_list == 0 ? group_row_capacity(hs[s].capacity) : hs[s].capacity))
+      if (req[s] > hs[s].capacity)
         throw Error(RMD_ERR_NEIGHBOUR_OVERFLOW,
                     "the neighbour list needed " + std::to_string(req[s]) + " slots per atom and the capacity is " +
                         std::to_string(hs[s].capacity) + ". Pairs were dropped, so the forces from this build are "
