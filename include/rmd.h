@@ -177,7 +177,9 @@ typedef struct {
   int32_t neighbour_required, neighbour_capacity, worst_neighbour_required, neighbour_growths;
   double skin, worst_displacement, worst_skin_ratio;
   int32_t skin_violations;
-  int64_t steps_with_stale_list;
+  int64_t steps_with_stale_list; /* steps of blocks whose forces may lack pairs: a displacement past the skin on the
+                                  * host's schedule, or a build inside the block that needed more than the rows
+                                  * hold (capacity; a quarter more with group-pair rows) */
   int32_t rebuild_interval, requested_rebuild_interval, rebuild_shrinks, rebuild_growths;
   double worst_skin_usage;
   int32_t adaptive_rebuild;

@@ -46,8 +46,9 @@ struct DevSys {
   long long nbr_base;   // offset of row 0 in the neighbour array
   int nbr_capacity;     // entries a per-atom row holds; more than this in any row makes the host grow the lists
   long long gnbr_base;  // offset of group slot 0's row in the group-pair array
-  // entries a group-pair row holds: a quarter more than nbr_capacity, so that a build inside a block of
-  // steps that passes it loses no pair before the host looks
+  // entries a group-pair row holds: a quarter more than nbr_capacity, so that a build inside a block of steps that
+  // needs up to that much loses no pair before the host grows the lists (one that needs more does, and the
+  // block's steps are counted in steps_with_stale_list)
   int gnbr_capacity;
   // Never written after the engine is built, and read by the spreading before it waits for its predecessor
   // (chain_begin): in a memory line that holds nothing else, because a line that such a read brings into a cache

@@ -167,6 +167,7 @@ struct HostSystem {
   int64_t steps_since_rebuild = 1LL << 40;
   double worst_displacement = 0, worst_skin_ratio = 0, worst_skin_usage = 0;
   int worst_required = 0, neighbour_growths = 0, last_required = 0;
+  bool pairs_dropped = false;  // some build since the last capacity check had rows too short
   bool kinetic_sampled_in_step = false;
   int64_t kinetic_sampled_at = -1;
   int n_clusters = 0, n_settle = 0;
@@ -1789,6 +1790,8 @@ int Engine::check_capacity() {
     hs[s].last_required = req[s];
     hs[s].worst_required = std::max(hs[s].worst_required, most);
     worst = std::max(worst, most);
+    // the rows the pair loop walks: a build that needed more than they hold left pairs out
+    hs[s].pairs_dropped = most > (pair_list == 1 ? hs[s].capacity : group_row_capacity(hs[s].capacity));
     if (most > hs[s].capacity) {
       hs[s].capacity = grown_capacity(hs[s].capacity, most);
       hs[s].neighbour_growths++;
@@ -2075,6 +2078,8 @@ void Engine::check_block(int steps) {
     h.steps_since_rebuild = 1LL << 40;
   }
   check_capacity();
+  for (HostSystem &h : hs)
+    if (h.pairs_dropped) h.steps_with_stale += steps;
 }
 
 void Engine::run(int64_t count, int block, const volatile int32_t *stop) {
