@@ -260,7 +260,7 @@ struct Engine {
   DevArray<FftZTask> tasks_z2;
   DevArray<FftPlaneTask> tasks_plane, tasks_cluster;
   std::vector<long long> recip_lo, recip_hi;  // per system range [lo, hi) of reciprocal energy partials
-  int fft_large = 0, z2_threads = 0, z2_smem = 0, plane_threads = 0, cluster_threads = 0;
+  int z2_large = 0, planes_large = 0, z2_threads = 0, z2_smem = 0, plane_threads = 0, cluster_threads = 0;
   int plane_stride = 0, cluster_rows = 0, cluster_cols = 0;
   DevArray<DevSys> sys;
   DevArray<DevSysD> sysd;
@@ -1090,7 +1090,6 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
       for (int ax = 0; ax < 3; ++ax) {
         for (double m : bspline_moduli(h.grid[ax], h.order)) h_mod.push_back((float)m);
         fft_axis_plan(h.grid[ax], h_plans[s].axis[ax], (int)h_tw.size());
-        if (h_plans[s].axis[ax].r2 > RADIX_SMALL) fft_large = 1;
         for (int k = 0; k < h.grid[ax]; ++k) {
           const double a = -2.0 * M_PI * k / h.grid[ax];
           h_tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
@@ -1107,6 +1106,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
           tz.push_back(FftTask{s, 0, p, std::min(mz, pairs - p)});
       }
       if (zax.r1 > 0) {
+        if (zax.r2 > RADIX_SMALL) z2_large = 1;
         z2_threads = std::max(z2_threads, std::min(256, (FFT_PAIRS_PER_BLOCK * zax.r2 + 31) / 32 * 32));
         z2_smem = std::max(z2_smem, FFT_PAIRS_PER_BLOCK * ((zax.r1 * (zax.r2 | 1)) | 1));
       }
@@ -1115,6 +1115,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
       // debug transforms run the separate passes over every system.
       split[s] = fft_plane_split(nx, ny);
       const bool fused = split[s] > 0;
+      if (fused && std::max(h_plans[s].axis[0].r2, h_plans[s].axis[1].r2) > RADIX_SMALL) planes_large = 1;
       // separate passes: y lines are the x rows of a plane, x lines its columns (padded to nx + 1)
       const int my = lines_per_block(all_ylines, ny, nx);
       const int mx = std::max(1, std::min(ny, std::min(FFT_SMEM_HOST / (nx + 1), 512 / (nx + 1))));
@@ -1476,7 +1477,8 @@ LaunchCtx Engine::ctx() const {
   c.fft_plans = fft_plans.p;
   c.tasks_z2 = tasks_z2.p;
   c.n_tasks_z2 = (int)tasks_z2.n;
-  c.fft_large = fft_large;
+  c.z2_large = z2_large;
+  c.planes_large = planes_large;
   c.z2_threads = z2_threads;
   c.z2_smem = z2_smem;
   c.plane_threads = plane_threads;

@@ -137,8 +137,12 @@ __device__ __forceinline__ void dft(float2 (&v)[R]) {
 }
 
 // Call f with the length, at most MAXR, as a compile-time constant. A kernel's registers are those
-// of its longest DFT, so the passes are built twice: for axes of factors up to RADIX_SMALL (every
-// axis up to 100 points and most up to 144) and for all.
+// of its longest DFT, so the passes are built twice: for axes of factors up to RADIX_SMALL (every axis up
+// to 144 points but 75, 125, 128 and 135) and for all. The longer form's blocks hold fewer to an SM (r2c 101 and
+// 254 registers a thread, planes 96 and 128 with some spilled), which shows beside its neighbours' times:
+// the reciprocal kernels of 42,000 atoms, us, against the Stockham passes that both replaced: 72^3 35 (66),
+// 75^3 41 (68), 80^3 38 (83); 120^3 72 (167), 125^3 119 (178), 128^3 70 (178), 135^3 90 (264), 144^3 89 (290), 150^3 135 (325),
+// 160^3 184 (261: its planes take the separate passes).
 constexpr int RADIX_SMALL = 12, RADIX_ALL = 25;
 template <int MAXR, class F>
 __device__ __forceinline__ void with_radix(int r, F &&f) {

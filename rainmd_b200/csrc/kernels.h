@@ -210,7 +210,7 @@ struct LaunchCtx {
   const FftPlaneTask *tasks_plane, *tasks_cluster;
   const FftTask *tasks_z, *tasks_y, *tasks_x, *tasks_y_all, *tasks_x_all;
   int n_tasks_z2, n_tasks_z, n_tasks_y, n_tasks_x, n_tasks_plane, n_tasks_cluster, n_tasks_y_all, n_tasks_x_all;
-  int fft_large;            // some axis has a factor above RADIX_SMALL
+  int z2_large, planes_large;  // some axis that the pass transforms has a factor above RADIX_SMALL
   int z2_threads, z2_smem;  // block size and complex values of shared memory of the two-factor z passes
   int plane_threads, cluster_threads;  // block sizes of the plane passes
   int plane_stride;  // complex values per plane buffer (the largest plane among the one-block systems)

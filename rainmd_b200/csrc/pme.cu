@@ -821,7 +821,7 @@ static void launch_forward_zy(const LaunchCtx &c, cudaStream_t stream, bool all 
   // last atomics land: the reciprocal kernels 33.1 -> 30.8 us at 64^3, 20.5 -> 17.9 at 24^3). The
   // generic pass stays a plain launch: chained it was slower at 64^3 (0.067 against 0.049 ms).
   if (c.n_tasks_z2 > 0)
-    launch_kernel(c.chain_pme, c.fft_large ? k_fft_r2c<RADIX_ALL> : k_fft_r2c<RADIX_SMALL>, c.n_tasks_z2, c.z2_threads,
+    launch_kernel(c.chain_pme, c.z2_large ? k_fft_r2c<RADIX_ALL> : k_fft_r2c<RADIX_SMALL>, c.n_tasks_z2, c.z2_threads,
                   c.z2_smem * sizeof(float2), stream, c.tasks_z2, c.twiddles, c.fixed_grid, c.half);
   if (c.n_tasks_z > 0)
     k_fft_z_r2c<<<c.n_tasks_z, 256, 0, stream>>>(c.tasks_z, c.sys, c.fft_plans, c.twiddles, c.fixed_grid, c.half);
@@ -835,8 +835,8 @@ static void launch_inverse_yz(const LaunchCtx &c, cudaStream_t stream, bool all 
   const int n = all ? c.n_tasks_y_all : c.n_tasks_y;
   if (n > 0) launch_kernel(c.chain_pme, k_fft_y, n, 256, 0, stream, ty, c.sys, c.fft_plans, c.twiddles, c.half, 1);
   if (c.n_tasks_z2 > 0)
-    launch_kernel(c.chain_pme, c.fft_large ? k_fft_c2r<RADIX_ALL> : k_fft_c2r<RADIX_SMALL>, c.n_tasks_z2, c.z2_threads, c.z2_smem * sizeof(float2), stream, c.tasks_z2,
-                  c.twiddles, c.half, c.real_grid);
+    launch_kernel(c.chain_pme, c.z2_large ? k_fft_c2r<RADIX_ALL> : k_fft_c2r<RADIX_SMALL>, c.n_tasks_z2, c.z2_threads,
+                  c.z2_smem * sizeof(float2), stream, c.tasks_z2, c.twiddles, c.half, c.real_grid);
   if (c.n_tasks_z > 0)
     launch_kernel(c.chain_pme, k_fft_z_c2r, c.n_tasks_z, 256, 0, stream, c.tasks_z, c.sys, c.fft_plans, c.twiddles,
                   c.half, c.real_grid);
@@ -918,8 +918,8 @@ static void launch_planes(const LaunchCtx &c, bool energy, cudaStream_t stream) 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = c.chain_pme ? 2 : 1;
-    auto kernel = c.fft_large ? (energy ? k_fft_planes<true, RADIX_ALL> : k_fft_planes<false, RADIX_ALL>)
-                              : (energy ? k_fft_planes<true, RADIX_SMALL> : k_fft_planes<false, RADIX_SMALL>);
+    auto kernel = c.planes_large ? (energy ? k_fft_planes<true, RADIX_ALL> : k_fft_planes<false, RADIX_ALL>)
+                                 : (energy ? k_fft_planes<true, RADIX_SMALL> : k_fft_planes<false, RADIX_SMALL>);
     (void)cudaLaunchKernelEx(&cfg, kernel, tasks, (const DevSys *)c.sys, c.twiddles, c.moduli, c.half, cl, rows, e, ev);
   };
   if (c.n_tasks_plane > 0) launch(1, c.tasks_plane, c.n_tasks_plane, c.plane_threads, c.plane_stride, 0);

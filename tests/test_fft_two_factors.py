@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from goldens import system_for
+from rainmd_b200.simulation import BatchSimulation
 from test_gpu_parity import ALPHA, engine_for, oracle_terms, relative
 
 pytestmark = pytest.mark.gpu
@@ -51,3 +52,24 @@ def test_z_passes_against_numpy(grid):
     assert np.max(np.abs(half - expect)) < bar
     assert np.max(np.abs(back / n - data.reshape(-1))) < 10 * 2 ** -24 * math.log2(n) * 4
     sim.release()
+
+
+def test_a_batch_gives_each_grid_its_own_bits():
+    """Axes of factors up to 12 and of longer ones take kernels built apart; which of them a system takes
+    depends on its own axes alone, whatever shares its handle."""
+    grids = [(64, 64, 64), (75, 75, 75), (24, 24, 24), (25, 75, 32), (160, 160, 8), (20, 24, 128), (125, 108, 16), (30, 30, 243)]
+    s, pos, _ = system_for("ala-wat")
+    options = [{"alpha": ALPHA, "grid": list(g), "skin": 0.1, "dispersionCorrection": False} for g in grids]
+    batch = BatchSimulation([s] * len(grids), options)
+    for k in range(len(grids)):
+        batch.setState(k, pos)
+    batch.initialise()
+    for k, g in enumerate(grids):
+        together, forces = batch.debugEvaluate(k)
+        sim = engine_for(s, pos, grid=list(g))
+        alone, expect = sim.debugEvaluate()
+        for term in ("coulomb_reciprocal", "potential", "volume_derivative"):
+            assert together[term] == alone[term], (g, term)
+        assert np.array_equal(forces, expect), g
+        sim.release()
+    batch.release()
