@@ -225,7 +225,7 @@ struct Engine {
   DevArray<float4> exc_param;
   DevArray<int> cell_of_atom, cell_count, cell_start, cell_atoms, cell_sys;
   int n_cells_total = 0;
-  DevArray<int> cell_gstart, group_order, group_sys;
+  DevArray<int> cell_gstart, cell_order, group_sys;
   int n_groups_total = 0;
   DevArray<int> nbr, nbr_count, required, required_max, stale;
   // group-pair rows (pair_list 0 and 2): rows, lengths, first order position and atoms per group
@@ -1015,7 +1015,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   cell_gstart.zero();
   n_groups_total = (int)h_group_sys.size();
   group_sys.upload(h_group_sys);
-  group_order.alloc(N);
+  cell_order.alloc(pair_list == 0 ? 1 : N);  // (only the per-atom search reads it)
   cell_atoms.alloc(N);
   cell_of_atom.alloc(N);
   spos.alloc(N);
@@ -1410,7 +1410,7 @@ LaunchCtx Engine::ctx() const {
   c.cell_sys = cell_sys.p;
   c.n_cells_total = n_cells_total;
   c.cell_gstart = cell_gstart.p;
-  c.group_order = group_order.p;
+  c.cell_order = cell_order.p;
   c.group_sys = group_sys.p;
   c.n_groups_total = n_groups_total;
   c.group_atoms = group_atoms;

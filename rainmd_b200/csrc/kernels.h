@@ -130,9 +130,10 @@ struct LaunchCtx {
   // lists
   int *cell_of_atom, *cell_count, *cell_start, *cell_atoms, *cell_sys;
   int n_cells_total;
-  // neighbour-search groups: per cell the first group (scan of ceil(count / 32), indexed like
-  // cell_start), the cell's slots in sub-cell order, and the system of each group slot
-  int *cell_gstart, *group_order;
+  // neighbour-search groups: per cell the first group (scan of ceil(count / group_atoms), indexed like
+  // cell_start), the order of the cell's atoms that the slots do not have (lists.cu LaunchCtxView), and the
+  // system of each group slot
+  int *cell_gstart, *cell_order;
   const int *group_sys;
   int n_groups_total;
   int group_atoms;  // atoms per neighbour-search group: 4, 8, 16 or 32

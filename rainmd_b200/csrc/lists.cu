@@ -27,7 +27,9 @@ struct LaunchCtxView {
   float4 *spos;
   float4 *wrap;
   int *sorted_orig, *sorted_type, *rank;
-  int *group_order;
+  // for the per-atom search (null when it does not run): slot of a cell's k-th atom in search order, or, where the
+  // slots are in search order themselves, of its k-th atom by index
+  int *cell_order;
   int2 *slot_info;  // per slot: LJ type, original index (the group-pair kernel's partner record)
   // group-pair rows only (else null): per 4-atom group slot its bounding box (lo, hi) of wrapped
   // positions, and the cell scan's first group per cell. The slots are then numbered in search
@@ -198,7 +200,7 @@ __device__ __forceinline__ int place_sorted(const LaunchCtxView &v, const DevSys
 // One block per allocated cell: rank-sort the cell's slice ascending, zero the cursor, write
 // the cell-ordered records of its atoms, and order the cell's atoms by sub-cell key (ties by
 // index), so that consecutive ones are spatially compact: into the slots themselves with
-// group-pair rows, else into group_order.
+// group-pair rows (cell_order then leads from the order by index to the slots), else into cell_order.
 __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__restrict__ sys,
                              const int *__restrict__ cell_start, int *__restrict__ cell_cursor,
                              int *__restrict__ cell_atoms, LaunchCtxView v, const int *__restrict__ only) {
@@ -251,9 +253,9 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
       const int rank = below(sub_keys, sub_keys[k]);
       if (by_group) {
         place_sorted(v, s, gbase + rank, sorted[k], cc);
-        v.group_order[gbase + k] = gbase + k;
+        if (v.cell_order) v.cell_order[gbase + k] = gbase + rank;
       } else {
-        v.group_order[gbase + rank] = gbase + k;
+        v.cell_order[gbase + rank] = gbase + k;
       }
     }
   } else {
@@ -272,7 +274,7 @@ __global__ void k_cells_sort(const int *__restrict__ cell_sys, const DevSys *__r
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       place_sorted(v, s, gbase + k, slice[k], cc);
-      v.group_order[gbase + k] = gbase + k;
+      if (v.cell_order) v.cell_order[gbase + k] = gbase + k;
     }
   }
   if (v.group_box) {  // the bounding box of each 4-atom group of this cell, for the search's cull
@@ -338,14 +340,21 @@ constexpr int NBR_SPLIT_GROUPS_MAX = 148 * 24 / 2;
 // of one long one, which fills the SMs when there are few groups. If a warp's hits overflow its
 // staging (512 per atom: a very dense neighbourhood) the first warp walks the whole stencil
 // again and writes the rows directly.
-template <int G, int SPLIT>
-__global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
+//
+// BY_GROUP: the slots are in search order (group-pair rows are built too), so a group's atoms are its slots
+// and cell_order gives a cell's candidates by index; otherwise the other way round. One kernel that asked at
+// each candidate and went through the atoms' indices to the slots: a rebuild without group-pair rows 1-5% longer
+// (3,000 atoms 176 us against 166), with them 275 against 213 at 3,000, 339 against 306 at 23,558 and 1,189 against
+// 1,069 at 99,999. Six blocks an SM (80 registers): left to itself the compiler takes 95 here and 240 us instead of 212 at
+// 23,558 atoms in groups of 4.
+template <int G, int SPLIT, bool BY_GROUP>
+__global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT, 6)
     k_neighbours(const float4 *__restrict__ posq, const int *__restrict__ group_sys,
                  const DevSys *__restrict__ sys, const int *__restrict__ cell_start,
-                 const int *__restrict__ cell_gstart, const int *__restrict__ group_order,
+                 const int *__restrict__ cell_gstart, const int *__restrict__ cell_order,
                  const int *__restrict__ excl_start, const int *__restrict__ excl_partners,
                  const float4 *__restrict__ spos, const int *__restrict__ sorted_orig,
-                 const int *__restrict__ cell_atoms, const int *__restrict__ rank, int *__restrict__ nbr, int *__restrict__ nbr_count, int *__restrict__ required,
+                 int *__restrict__ nbr, int *__restrict__ nbr_count, int *__restrict__ required,
                  float4 *__restrict__ origin, int n_groups, const int *__restrict__ only) {
   constexpr int J = 32 / G;
   constexpr int WARPS = SPLIT == 1 ? NBR_WARPS : SPLIT;
@@ -380,7 +389,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
   const int cend = s.atom_start + cell_start[s.cell_start_base + cell0 + 1];
   const int k = cbegin + (q - gstart[cell0]) * G + a;
   const bool valid = k < cend;
-  const int si = valid ? group_order[k] : -1;
+  const int si = valid ? (BY_GROUP ? k : cell_order[k]) : -1;
   const int i = valid ? sorted_orig[si] : 0;
   const float4 pw = valid ? spos[si] : make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid && sub == 0 && (SPLIT == 1 || wib == 0)) origin[i] = posq[i];  // skin check origin
@@ -468,7 +477,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT)
             bool keep = g < end;
             float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
             if (keep) {
-              if (cell_atoms) g = rank[cell_atoms[g]];  // slots in search order: the g-th atom by index
+              if (BY_GROUP) g = cell_order[g];
               pj = spos[g];
               if (stencil_shift) {  // drop candidates beyond the list cutoff from the bounding box
                 const float c[3] = {pj.x, pj.y, pj.z};
@@ -900,7 +909,7 @@ void launch_rebuild(const LaunchCtx &ctx, cudaStream_t stream) {
                                                          ctx.cell_start, ctx.cell_count,
                                                          ctx.cell_atoms, n, only);
   LaunchCtxView v{ctx.posq,      ctx.atom_type, ctx.spos,      ctx.wrap,      ctx.sorted_orig,
-                  ctx.sorted_type, ctx.rank,   ctx.group_order, ctx.slot_info,
+                  ctx.sorted_type, ctx.rank,   ctx.pair_list == 0 ? nullptr : ctx.cell_order, ctx.slot_info,
                   ctx.pair_list != 1 ? ctx.group_box : nullptr, ctx.cell_gstart, ctx.group_cell};
   k_cells_sort<<<ctx.n_cells_total, 256, 0, stream>>>(ctx.cell_sys, ctx.sys, ctx.cell_start,
                                                       ctx.cell_count, ctx.cell_atoms, v, only);
@@ -916,25 +925,27 @@ void launch_rebuild(const LaunchCtx &ctx, cudaStream_t stream) {
     if (n_groups >= GROUP_ROW_WARP_GROUPS) rows(k_group_rows<1>, (n_groups + 3) / 4, 128);
     else if (n_groups >= GROUP_ROW_BLOCK_GROUPS) rows(k_group_rows<4>, n_groups, 128);
     else rows(k_group_rows<8>, n_groups, 256);
-    if (ctx.pair_list != 2) return;
   }
-#define RMD_NBR_ARGS                                                                                      \
-  ctx.posq, ctx.group_sys, ctx.sys, ctx.cell_start, ctx.cell_gstart, ctx.group_order, ctx.excl_start,  \
-      ctx.excl_partners, ctx.spos, ctx.sorted_orig, ctx.pair_list == 2 ? ctx.cell_atoms : nullptr, ctx.rank, ctx.nbr, ctx.nbr_count, ctx.required, ctx.origin, \
-      ctx.n_groups_total, only
+  if (ctx.pair_list == 0) return;
+  auto search = [&](auto kernel, int blocks, int threads) {
+    kernel<<<blocks, threads, 0, stream>>>(ctx.posq, ctx.group_sys, ctx.sys, ctx.cell_start, ctx.cell_gstart,
+                                           ctx.cell_order, ctx.excl_start, ctx.excl_partners, ctx.spos, ctx.sorted_orig,
+                                           ctx.nbr, ctx.nbr_count, ctx.required, ctx.origin, ctx.n_groups_total, only);
+  };
+  const bool by_group = ctx.pair_list == 2;  // (4-atom groups)
   // 4-atom groups too few to fill the GPU with one warp each (a box of a few thousand atoms)
   // search three warps a group; otherwise one warp a group keeps more groups resident
   if (G == 4 && ctx.n_groups_total < NBR_SPLIT_GROUPS_MAX)
-    k_neighbours<4, NBR_SPLIT><<<ctx.n_groups_total, 32 * NBR_SPLIT, 0, stream>>>(RMD_NBR_ARGS);
+    search(by_group ? k_neighbours<4, NBR_SPLIT, true> : k_neighbours<4, NBR_SPLIT, false>, ctx.n_groups_total,
+           32 * NBR_SPLIT);
   else if (G == 4)
-    k_neighbours<4, 1><<<blocks, 32 * NBR_WARPS, 0, stream>>>(RMD_NBR_ARGS);
+    search(by_group ? k_neighbours<4, 1, true> : k_neighbours<4, 1, false>, blocks, 32 * NBR_WARPS);
   else if (G == 8)
-    k_neighbours<8, 1><<<blocks, 32 * NBR_WARPS, 0, stream>>>(RMD_NBR_ARGS);
+    search(k_neighbours<8, 1, false>, blocks, 32 * NBR_WARPS);
   else if (G == 16)
-    k_neighbours<16, 1><<<blocks, 32 * NBR_WARPS, 0, stream>>>(RMD_NBR_ARGS);
+    search(k_neighbours<16, 1, false>, blocks, 32 * NBR_WARPS);
   else
-    k_neighbours<32, 1><<<blocks, 32 * NBR_WARPS, 0, stream>>>(RMD_NBR_ARGS);
-#undef RMD_NBR_ARGS
+    search(k_neighbours<32, 1, false>, blocks, 32 * NBR_WARPS);
 }
 
 }  // namespace rmd
