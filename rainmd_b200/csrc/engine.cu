@@ -547,7 +547,7 @@ static void fft_axis_plan(int n, FftAxis &ax, int tw_base) {
 }
 
 static FftTwo fft_two(const FftAxis &ax) {
-  return FftTwo{ax.n, ax.r1, ax.r2, ax.tw_base, make_fast_div((uint32_t)ax.r1), make_fast_div((uint32_t)ax.r2), ax.n_div};
+  return FftTwo{ax.n, ax.r1, ax.r2, ax.tw_base, make_fast_div((uint32_t)ax.r1), make_fast_div((uint32_t)ax.r2)};
 }
 
 constexpr int FFT_SMEM_HOST = 2048;
@@ -1137,8 +1137,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
         const FftTwo x = fft_two(h_plans[s].axis[0]), y = fft_two(h_plans[s].axis[1]);
         planes.push_back(FftPlaneTask{d.half_base + (long long)kz * nx * ny, s, kz, nz, d.moduli_base, threads, x, y,
                                       make_fast_div((uint32_t)((nx + split[s] - 1) / split[s])),
-                                      make_fast_div((uint32_t)((ny + split[s] - 1) / split[s])),
-                                      make_fast_div((uint32_t)(y.r1 * (y.r2 | 1)))});
+                                      make_fast_div((uint32_t)((ny + split[s] - 1) / split[s]))});
       }
       if (split[s] == 1) {
         plane_stride = std::max(plane_stride, rows);

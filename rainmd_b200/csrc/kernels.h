@@ -35,7 +35,7 @@ struct FftPlan {
 // plan, so it is one read, and nothing in it changes after the engine is built.
 struct FftTwo {
   int n, r1, r2, tw_base;
-  FastDiv r1_div, r2_div, n_div;
+  FastDiv r1_div, r2_div;
 };
 struct FftZTask {
   long long grid_base, half_base;
@@ -46,7 +46,7 @@ struct FftPlaneTask {
   long long half_base;      // of this kz plane
   int sys, kz, nz, moduli_base, threads;
   FftTwo x, y;
-  FastDiv rows_div, cols_div, ldy_div;  // rows and columns a block of the cluster; a row's padded length
+  FastDiv rows_div, cols_div;  // rows and columns a block of the cluster
 };
 constexpr int FFT_TWO_MAX = 400;          // longest axis of the two-factor passes (20 x 20)
 constexpr int FFT_PAIRS_PER_BLOCK = 8;    // pairs of real z lines a two-factor z block transforms
