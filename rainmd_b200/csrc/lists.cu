@@ -306,8 +306,11 @@ __device__ __forceinline__ bool is_excluded(const int *__restrict__ start, const
   return false;
 }
 
-// Group slots from which a warp builds a row alone, and from which four warps do instead of eight.
-constexpr int GROUP_ROW_WARP_GROUPS = 148 * 64 * 2;
+// Group slots from which a warp builds a row alone, and from which four warps do instead of eight: each where
+// the form with fewer warps a row has one full wave of blocks (eight an SM, of four rows or of one). A rebuild with
+// one / four / eight warps a row, us: 633 slots 89 / 59 / 53; 883 95 / 65 / 66; 1,008 100 / 72 / 75; 1,278 74 / 45 / 48;
+// 2,277 92 / 68 / 81; 4,064 92 / 86 / 107; 6,015 82 / 96 / 125; 9,591 118 / 144 / 192; 15,343 152 / 203 / 285; 23,012 201 / 283 / 407.
+constexpr int GROUP_ROW_WARP_GROUPS = 148 * 8 * 4;
 constexpr int GROUP_ROW_BLOCK_GROUPS = 148 * 8;
 constexpr int NBR_WARPS = 4;        // groups per block when one warp searches for a group
 constexpr int NBR_SPLIT = 3;        // warps per group in the split search (one stencil x-slab each)
@@ -607,7 +610,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT, 6)
 }
 
 // ---------------------------------------------------------------- group-pair rows
-// One WARP per search group of GROUP_ATOMS atoms (the groups of k_neighbours<4, 1>): the
+// One, four or eight warps per search group of GROUP_ATOMS atoms (the groups of k_neighbours<4, 1>): the
 // group's row lists every partner atom that lies within the list cutoff of one of the group's
 // atoms through some lattice image, once per such image, and only if the pair belongs
 // to this group: the partner comes later in search order (its slot is beyond the group's), or it
@@ -632,9 +635,9 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT, 6)
 // walks instead of one long one; with enough groups to fill the GPU a warp a row does the same with
 // less work. The order of a row's entries then depends on the warps' timing; its contents do not, and
 // neither does any force (every pair's fixed-point force is added whatever the order). The rebuild's
-// kernels, before and with this form: 250,000 atoms (a warp a row) 814 -> 512 us, 99,999 353 -> 238, a
-// batch of 24 systems 417 -> 218, 23,558 (four warps) 107 -> 101, 2,854 and 1,190 (eight, most visits
-// dropped) 92 -> 61 and 68 -> 40.
+// kernels, before and with this form: 250,000 atoms (a warp a row) 814 -> 512 us, 99,999 353 -> 231, a
+// batch of 24 systems 417 -> 218, 23,558 107 -> 82, 9,000 (four warps) 72 -> 68, 2,854 and 1,190 (eight, most visits
+// dropped) 92 -> 59 and 68 -> 40.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS == 1 ? 128 : 32 * WARPS, WARPS == 8 ? 4 : 8)
     k_group_rows(const float4 *__restrict__ posq, const int *__restrict__ group_sys,
