@@ -329,7 +329,9 @@ __device__ __forceinline__ void group_pair_entry(const unsigned e, const float4 
   }
 }
 
-constexpr int PREFETCH_GROUPS = 48 * 1024;  // groups whose rows together pass about 80 MB
+// Groups whose rows together (1.7 KB each at a skin of 0.25 nm) pass some 60 MB: a part of them is then read from device
+// memory in each step.
+constexpr int PREFETCH_GROUPS = 36 * 1024;
 
 template <bool ENERGY>
 __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
@@ -367,8 +369,8 @@ __global__ void __launch_bounds__(128, ENERGY ? 4 : 5) k_group_pairs(
   const int wib = threadIdx.x >> 5;
   const int *row = gnbr + s.gnbr_base + (long long)(warp - s.group_base) * s.gnbr_capacity;
   // Rows too many for L2 are read from device memory: this one starts on its way while the records
-  // below are read (250,000 atoms 354 -> 341 us; 99,999 143.0 -> 143.9 and a batch 112.6 -> 114, whose
-  // rows stay in L2, hence the line).
+  // below are read. Without / with, us: 15,343 group slots 87.3 / 88.1; 25,512 141.6 / 142.4; 30,729 168.0 / 167.9; 38,229
+  // 211.9 / 209.3; 43,500 242.9 / 237.9; 63,831 345 / 335; 76,728 428 / 413; hence the line.
   if (n_groups >= PREFETCH_GROUPS)
     for (int k = 32 * lane; k < count; k += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + k));
   if (lane < 27) shift[wib][lane] = s.shift[lane];
