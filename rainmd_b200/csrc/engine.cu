@@ -228,8 +228,8 @@ struct Engine {
   DevArray<int> cell_gstart, cell_order, group_sys;
   int n_groups_total = 0;
   DevArray<int> nbr, nbr_count, required, required_max, stale;
-  // group-pair rows (pair_list 0 and 2): rows, lengths, first order position and atoms per group
-  // slot; per slot its partner record and order position; per-atom integer energy sums
+  // group-pair rows (pair_list 0 and 2): rows, lengths, first slot, atoms, cell and box per group
+  // slot; per slot its partner record; per-atom integer energy sums
   int pair_list = 1;
   DevArray<int> gnbr, gnbr_count, gfirst, gsize, group_cell;
   DevArray<float4> group_box;
@@ -2293,8 +2293,8 @@ std::vector<float> Engine::max_forces() {
 
 // minimise (simulation.js:880-979): steepest descent with a backtracking line search. Every
 // system of a batch keeps its own step and acceptance, and every decision is taken on the
-// device (minimise.cu): one trial is one captured graph, launched in batches of 16 with the
-// states read back between batches. A trial whose neighbour list overflowed is undone on the
+// device (minimise.cu): one trial is one captured graph, launched in batches of 2 to 16 (by the
+// iterations left) with the states read back between batches. A trial whose neighbour list overflowed is undone on the
 // device; the host grows the list, re-captures and the trial runs again.
 // Departure: the positions AND forces of the last accepted structure are restored after a
 // rejected trial, so the next trial moves along the accepted gradient.

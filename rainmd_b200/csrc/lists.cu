@@ -8,10 +8,13 @@
 //   - the histogram and the scatter use integer atomics, and a per-cell block rank-sort
 //     (shared memory) restores the deterministic index order;
 //   - the scan is one block per system;
-//   - the neighbour search is one WARP per group of 4, 8, 16 or 32 spatially close atoms of a
-//     cell: the group's bounding box culls stencil cells and candidates once for all its
-//     atoms, the survivors are staged in shared memory, and each atom's lanes append its
-//     hits in candidate order, so every row's order equals the sequential one.
+//   - the per-atom search (pair_list 1 and 2) is one WARP per group of 4, 8, 16 or 32 spatially
+//     close atoms of a cell, or three for small launches: the group's bounding box culls stencil cells
+//     and candidates once for all its atoms, the survivors are staged in shared memory, and each
+//     atom's lanes append its hits in candidate order, so every row's order equals the
+//     sequential one;
+//   - the rows that the pair kernel walks by default (pair_list 0 and 2) are half lists of 4-atom
+//     groups, built by one, four or eight warps a group in no particular order (k_group_rows).
 #include <climits>
 
 #include <algorithm>

@@ -126,9 +126,9 @@ __device__ __forceinline__ int wrap_near(int v, int n) {
 // threads of a ky add consecutive z points together: a warp's atomic instruction covers rows of
 // 8 * ORDER bytes, one or two sectors each, where a thread a (kx, ky) touched 32 sectors an
 // instruction. Each thread recomputes the atom's splines (cheap) so no cross-thread exchange is
-// needed. Bound by the L2's atomics. With the
-// gather's wrapped indices below, the reciprocal kernels at 250,000 atoms on 144^3 went from 170 to
-// 133 us, at 23,558 on 64^3 from 38.2 to 32.8.
+// needed. With the gather's wrapped indices below, the reciprocal kernels at 250,000 atoms on 144^3 went from
+// 170 to 133 us, at 23,558 on 64^3 from 38.2 to 32.8. At 23,558 atoms (9.7 us cold, 14.2 before) its warps wait for
+// the atoms' records (long scoreboard 9.7 of them an issue); the L2's atomic input is busy 19% of the time.
 template <int ORDER>
 __global__ void k_spread(const float4 *__restrict__ posq, const int *__restrict__ sys_of_atom,
                          const DevSys *__restrict__ sys, unsigned long long *__restrict__ fixed_grid,
