@@ -310,9 +310,10 @@ __device__ __forceinline__ bool is_excluded(const int *__restrict__ start, const
 }
 
 // Group slots from which a warp builds a row alone, and from which four warps do instead of eight: each where
-// the form with fewer warps a row has one full wave of blocks (eight an SM, of four rows or of one). A rebuild with
-// one / four / eight warps a row, us: 633 slots 89 / 59 / 53; 883 95 / 65 / 66; 1,008 100 / 72 / 75; 1,278 74 / 45 / 48;
-// 2,277 92 / 68 / 81; 4,064 92 / 86 / 107; 6,015 82 / 96 / 125; 9,591 118 / 144 / 192; 15,343 152 / 203 / 285; 23,012 201 / 283 / 407.
+// the form with fewer warps a row has one full wave of blocks (eight an SM, of four rows or of one). A rebuild of
+// water after 200 steps with one / four / eight warps a row, us: 633 slots 90 / 58 / 53; 883 94 / 64 / 65; 1,152 74 / 45 / 45;
+// 1,278 79 / 47 / 49; 2,277 91 / 68 / 80; 4,064 94 / 87 / 109; 4,564 103 / 98 / 125; 5,125 80 / 84 / 109; 6,015 87 / 99 / 129; 9,591 125 /
+// 150 / 198; 15,343 161 / 212 / 293; batches of 4,727 slots 82 / 85 / 105 and of 5,030 100 / 123 / 161.
 constexpr int GROUP_ROW_WARP_GROUPS = 148 * 8 * 4;
 constexpr int GROUP_ROW_BLOCK_GROUPS = 148 * 8;
 constexpr int NBR_WARPS = 4;        // groups per block when one warp searches for a group
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 32 * NBR_WARPS : 32 * SPLIT, 6)
 // less work. The order of a row's entries then depends on the warps' timing; its contents do not, and
 // neither does any force (every pair's fixed-point force is added whatever the order). The rebuild's
 // kernels, before and with this form: 250,000 atoms (a warp a row) 814 -> 512 us, 99,999 353 -> 231, a
-// batch of 24 systems 417 -> 218, 23,558 107 -> 82, 9,000 (four warps) 72 -> 68, 2,854 and 1,190 (eight, most visits
+// batch of 24 systems 417 -> 214, 23,558 107 -> 95, 9,000 (four warps) 72 -> 68, 2,854 and 1,190 (eight, most visits
 // dropped) 92 -> 59 and 68 -> 40.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS == 1 ? 128 : 32 * WARPS, WARPS == 8 ? 4 : 8)
