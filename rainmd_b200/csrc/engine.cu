@@ -380,7 +380,9 @@ struct Engine {
   // is one asynchronous transfer on the engine stream, and the call waits once.
   void *pinned = nullptr;
   size_t pinned_bytes = 0;
+  size_t staging_least = 0;  // what a setState or readState of the largest system takes: allocated at the first use
   char *staging(size_t bytes) {
+    bytes = std::max(bytes, staging_least);
     if (bytes > pinned_bytes) {
       if (pinned) CUDA_OK(cudaFreeHost(pinned));
       pinned = nullptr;
@@ -1035,6 +1037,7 @@ void Engine::upload_all(const std::vector<const rmd_system *> &src) {
   int largest = 0;
   for (auto &h : hs) largest = std::max(largest, h.n);
   state_out.alloc(9 * (size_t)largest);
+  staging_least = 9 * sizeof(float) * (size_t)largest + sizeof(DevSysD);
   allocate_status();
   stale.alloc(S);
   stale.zero();
